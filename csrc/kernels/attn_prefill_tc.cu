@@ -1,12 +1,392 @@
-// Prefill attention over the paged cache, heads of 64 or 128 (see attn_prefill_tc.cuh).
+// Prefill attention over the paged cache, heads of 64 or 128: pairs of query heads that share a key head
+// (below), one head per CTA where a key head has an odd number of them (attn_prefill_tc.cuh).
 #include "attn_prefill_tc.cuh"
 
 namespace oxb {
+
+namespace {
+
+// Two query heads of one key head per CTA. With one head per CTA (attn_prefill_tc.cuh) the tensor core waits for the
+// softmax of the only tile in flight and the softmax for its scores: 463 TFLOP/s at 8192 queries behind 24576 positions,
+// 8 x 4 heads of 128 (8319 us). Here two softmax groups of 128 threads take turns with the tensor core: while one group works
+// on its scores, the products of the other run. A pair of heads has the same keys, values and masks, so a KV tile is
+// fetched once for both. P goes back to TMEM over the scores it was made of (tcgen05.mma with A in TMEM): it
+// needs no shared memory, which holds a ring of K and V tiles, and one commit orders everything: MMAs run in issue
+// order, so when S(j + 1) is complete, P(j) V is too, and P and O of that head may be written. 1010 TFLOP/s (3799 us) at the
+// same sizes, 302 -> 123 us for 14 prompts of 128 to 1024 tokens; what bounds it now is the exponentials (16 per clock and SM, as
+// long as the two products of a tile) and the scores' operands, which take all of the shared-memory bandwidth while they run.
+template <int D, bool EXACT>
+struct PairSmem {
+  static constexpr int kHalves = D / 64;
+  static constexpr int kSlotBytes = kHalves * kHalfBytes;      // one [128 x D] tile of K or V
+  static constexpr int kSlots = D == 128 ? 5 : 8;              // K and V tiles in flight: K(0) V(0) K(1) V(1) ...
+  static constexpr int kQ = 0;                                 // [2 heads][128 x D]
+  static constexpr int kRing = 2 * kSlotBytes;
+  static constexpr int kBar = kRing + kSlots * kSlotBytes;
+  static constexpr int kTotal = kBar + 256 + 1024;
+};
+
+// Warpgroup 0: producer warp, MMA warp and two idle ones; warpgroups 1 and 2: softmax. A row of 128 scores is held in
+// registers, so the softmax threads take over registers of the first group: 72 + 2 x 216 = 3 x 168 as launched.
+constexpr int kPairThreads = 384;
+constexpr int kIssueRegs = 72, kSoftmaxRegs = 216;
+static_assert(kIssueRegs + 2 * kSoftmaxRegs <= 3 * 168, "register split");
+
+template <int D, bool EXACT>
+__global__ void __launch_bounds__(kPairThreads, 1)
+prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                    const __grid_constant__ CUtensorMap tmV, const PrefillAttnParams p, int* status) {
+  using L = PairSmem<D, EXACT>;
+  constexpr int BKV = 128, KH = L::kHalves, NS = L::kSlots;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sQ = smem + L::kQ;
+  uint8_t* ring = smem + L::kRing;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBar);
+  uint64_t* q_full = bars;
+  uint64_t* full = bars + 1;           // [NS]
+  uint64_t* empty = full + NS;         // [NS]
+  uint64_t* s_full = empty + NS;       // [2] scores of a head are complete
+  uint64_t* p_full = s_full + 2;       // [2] its softmax weights are in TMEM
+  uint64_t* o_full = p_full + 2;       // [2] its last value product is complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+
+  // late tiles see the longest contexts: they go first
+  const int tile = gridDim.x - 1 - blockIdx.x;
+  const int head0 = 2 * blockIdx.y;
+  const int q0 = p.tile_q0[tile];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int seq = p.tile_seq[tile];
+  const int q_len = p.q_lens[seq];
+  const int ctx = p.ctx_lens[seq];
+  const int row_base = p.q_start[seq];
+  const int pos_off = ctx - q_len;
+  const int kvh = head0 / (p.Hq / p.Hkv);
+
+  int last_row = q0 + BQ - 1;
+  if (last_row > q_len - 1) last_row = q_len - 1;
+  const int max_pos = pos_off + last_row;
+  auto visible_from = [&](int pos) -> int {
+    if (p.chunk > 0) return pos / p.chunk * p.chunk;
+    return p.window > 0 ? pos - p.window + 1 : 0;
+  };
+  int first_tile = visible_from(pos_off + q0) / BKV;
+  if (first_tile < 0) first_tile = 0;
+  // the tiles with kept first positions come first, then the window's: entry j is tile j + (j < n_first ? 0 : skip)
+  int n_first = 0;
+  if (p.keep_first > 0 && first_tile > 0) {
+    n_first = (p.keep_first + BKV - 1) / BKV;
+    if (n_first > first_tile) n_first = first_tile;
+  }
+  const int skip = first_tile - n_first;
+  const int n_tiles = max_pos / BKV + 1 - skip;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+    mbar_init(q_full, 1);
+    for (int i = 0; i < NS; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&p_full[i], 4);
+      mbar_init(&o_full[i], 1);
+    }
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  // columns [0, 128), [128, 256): scores of the two heads, then their weights; from 256 on the two accumulators of D columns
+
+  if (warp < 4) {
+    warpgroup_regs_dec<kIssueRegs>();
+    if (warp == 0) {
+      // ------------------------------ TMA producer ------------------------------
+      // One lane per box of 16 rows x 64 columns of a KV tile: copies issued by one thread complete about one per memory
+      // round trip, copies of several threads run side by side.
+      if (lane == 0) mbar_arrive_expect_tx(q_full, 2 * L::kSlotBytes);
+      __syncwarp();
+      if (lane < 2 * KH)
+        tma_load_2d(sQ + lane * kHalfBytes, &tmQ, q_full, head0 * D + lane * 64, row_base + q0);
+      const int* bt = p.block_tables + static_cast<long long>(seq) * p.max_blocks;
+      const int pg = lane / KH, hf = lane % KH;  // this lane's page of a tile and its 64 columns
+      auto page = [&](int j) -> int {
+        const int pi = (j < n_first ? j : j + skip) * (BKV / 16) + pg;
+        return lane < KH * (BKV / 16) && j < n_tiles && pi < p.max_blocks ? bt[pi] : 0;
+      };
+      bool ok = true;
+      int next = page(0);
+      uint32_t item = 0;
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        int blk = next;
+        next = page(j + 1);
+        if (p.num_blocks > 0 && static_cast<unsigned>(blk) >= static_cast<unsigned>(p.num_blocks)) {
+          set_status_once(status, kStatusBadIndex);
+          blk = 0;
+        }
+        const int row = (blk * p.Hkv + kvh) * 16;
+        for (int v = 0; v < 2; ++v, ++item) {
+          const int s = item % NS;
+          if (item >= NS && !mbar_wait(&empty[s], (item / NS - 1) & 1)) ok = false;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) {
+            if (lane == 0) set_status_once(status, kStatusMbarTimeoutProducer);
+            break;
+          }
+          if (lane == 0) mbar_arrive_expect_tx(&full[s], L::kSlotBytes);
+          __syncwarp();
+          if (lane < KH * (BKV / 16))
+            tma_load_2d(ring + s * L::kSlotBytes + hf * kHalfBytes + pg * 2048, v ? &tmV : &tmK, &full[s], hf * 64, row);
+        }
+      }
+    } else if (warp == 1) {
+      // ------------------------------ MMA issuer --------------------------------
+      if (lane == 0) {
+        constexpr uint32_t idesc_s = make_idesc(kFmtBF16, kFmtBF16, BQ, BKV);
+        constexpr uint32_t idesc_o = make_idesc(kFmtBF16, kFmtBF16, BQ, D, 0, 1);  // V is MN-major
+        bool ok = mbar_wait(q_full, 0);
+        auto issue_s = [&](int g, uint32_t k_item) {
+          const uint32_t qa = smem_u32(sQ) + g * L::kSlotBytes;
+          const uint32_t kb = smem_u32(ring) + (k_item % NS) * L::kSlotBytes;
+  #pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t at = (kk >> 2) * kHalfBytes + (kk & 3) * 32;
+            tc_mma_f16(tmem_base + g * 128, make_desc_kmajor_sw128(qa + at), make_desc_kmajor_sw128(kb + at), idesc_s,
+                       kk != 0 ? 1u : 0u);
+          }
+          tc_commit(&s_full[g]);
+        };
+        if (ok && n_tiles > 0) {
+          ok = mbar_wait(&full[0], 0);
+          tc_fence_after_sync();
+          if (ok) {
+            issue_s(0, 0);
+            issue_s(1, 0);
+            tc_commit(&empty[0]);
+          }
+        }
+        for (int j = 0; j < n_tiles && ok; ++j) {
+          const uint32_t v_item = 2 * j + 1, k_item = 2 * j + 2;
+          ok = mbar_wait(&full[v_item % NS], (v_item / NS) & 1);
+          for (int g = 0; g < 2 && ok; ++g) {
+            if (!mbar_wait(&p_full[g], j & 1)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after_sync();
+            const uint32_t vb = smem_u32(ring) + (v_item % NS) * L::kSlotBytes;
+            const uint32_t pa = tmem_base + g * 128, od = tmem_base + 256 + g * D;
+  #pragma unroll
+            for (int kk = 0; kk < BKV / 16; ++kk)
+              tc_mma_f16_ts(od, pa + kk * 8, make_desc_mnmajor_sw128(vb + kk * 2048, kHalfBytes, 1024), idesc_o,
+                            (j | kk) != 0 ? 1u : 0u);
+            if constexpr (EXACT) {
+  #pragma unroll
+              for (int kk = 0; kk < BKV / 16; ++kk)
+                tc_mma_f16_ts(od, pa + 64 + kk * 8, make_desc_mnmajor_sw128(vb + kk * 2048, kHalfBytes, 1024), idesc_o, 1u);
+            }
+            if (g == 1) tc_commit(&empty[v_item % NS]);
+            if (j + 1 < n_tiles) {
+              if (g == 0) ok = mbar_wait(&full[k_item % NS], (k_item / NS) & 1);
+              if (!ok) break;
+              tc_fence_after_sync();
+              issue_s(g, k_item);
+              if (g == 1) tc_commit(&empty[k_item % NS]);
+            } else {
+              tc_commit(&o_full[g]);
+            }
+          }
+        }
+        if (!ok) set_status_once(status, kStatusMbarTimeoutMma);
+      }
+    }
+  } else {
+    warpgroup_regs_inc<kSoftmaxRegs>();
+    // ------------------------------ softmax + epilogue ------------------------
+    const int g = (warp - 4) >> 2;  // head of this group
+    const int q = warp & 3;
+    const int r = q * 32 + lane;  // query row of this thread == TMEM lane
+    const int head = head0 + g;
+    const int qi = q0 + r;
+    const bool row_valid = qi < q_len;
+    const int pos = pos_off + (row_valid ? qi : q_len - 1);
+    const int lo = visible_from(pos);
+    const int hi_lo = visible_from(max_pos);  // a tile between here and the first query's position needs no mask
+    const uint32_t lane_sel = static_cast<uint32_t>(q * 32) << 16;
+    const uint32_t s_addr = tmem_base + g * 128 + lane_sel;
+    const uint32_t o_addr = tmem_base + 256 + g * D + lane_sel;
+    float m_used = -INFINITY;
+    float2 l2 = make_float2(0.f, 0.f);
+    bool ok = true;
+    for (int j = 0; j < n_tiles; ++j) {
+      if (ok && !mbar_wait(&s_full[g], j & 1)) ok = false;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after_sync();
+      const int t0 = (j < n_first ? j : j + skip) * BKV;
+      uint32_t v[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32b_x32(s_addr + c * 32, v[c]);
+      tmem_ld_wait();
+      if (t0 + BKV - 1 > pos_off + q0 || t0 < hi_lo) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const int t = t0 + c * 32 + i;
+            const bool keep = t <= pos && (t >= lo || t < p.keep_first);
+            if (!keep) v[c][i] = 0xFF800000u;  // -infinity
+          }
+      }
+      float mx4[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        mx4[c] = __uint_as_float(v[c][0]);
+#pragma unroll
+        for (int i = 1; i < 31; i += 2)
+          mx4[c] = fmaxf(fmaxf(mx4[c], __uint_as_float(v[c][i])), __uint_as_float(v[c][i + 1]));
+        mx4[c] = fmaxf(mx4[c], __uint_as_float(v[c][31]));
+      }
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+      // the maximum is followed lazily: O is rescaled only when a row's grows by more than 2^8
+      float alpha = 1.f;
+      bool grow = false;
+      if (mx > m_used + 8.f || (m_used == -INFINITY && mx > -INFINITY)) {
+        alpha = m_used == -INFINITY ? 0.f : ex2a(m_used - mx);
+        m_used = mx;
+        grow = true;
+      }
+      if (j > 0 && __any_sync(0xffffffffu, grow)) {
+        // these scores are complete, so is every product issued before them: O is at rest
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld_32x32b_x32(o_addr + c * 32, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st_32x32b_x32(o_addr + c * 32, o);
+        }
+        l2.x *= alpha;
+        l2.y *= alpha;
+      }
+      const float m_sub = m_used == -INFINITY ? 0.f : m_used;
+      const float2 sc = make_float2(p.scale_log2, p.scale_log2), off = make_float2(-m_sub, -m_sub);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t w[32], wl[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const int c = 2 * h + (i >> 4), e = (2 * i) & 31;
+          float2 x = fma_f32x2(make_float2(__uint_as_float(v[c][e]), __uint_as_float(v[c][e + 1])), sc, off);
+          x.x = ex2a(x.x);
+          x.y = ex2a(x.y);
+          l2 = add_f32x2(l2, x);
+          w[i] = pack_bf16x2(x.x, x.y);
+          if constexpr (EXACT)
+            wl[i] = pack_bf16x2(x.x - __uint_as_float(w[i] << 16), x.y - __uint_as_float(w[i] & 0xFFFF0000u));
+        }
+        tmem_st_32x32b_x32(s_addr + h * 32, w);
+        if constexpr (EXACT) tmem_st_32x32b_x32(s_addr + 64 + h * 32, wl);
+      }
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[g]);
+    }
+    // ---- epilogue: O / l -> rows ----
+    if (ok && n_tiles > 0) {
+      if (!mbar_wait(&o_full[g], 0)) ok = false;
+      ok = __all_sync(0xffffffffu, ok);
+    }
+    if (!ok && lane == 0) set_status_once(status, kStatusMbarTimeoutEpilogue);
+    if (ok && n_tiles > 0) {
+      tc_fence_after_sync();
+      float l_sum = l2.x + l2.y;
+      const float sink = p.sinks != nullptr ? p.sinks[head] * 1.4426950408889634f : p.sink_log2;
+      if (sink != -INFINITY) l_sum += ex2a(sink - m_used);
+      const float inv = l_sum > 0.f ? p.out_gain / l_sum : 0.f;
+      const int od = p.out_d > 0 ? p.out_d : D;  // values stored per head
+      const bool vec = (od & 7) == 0 && (p.out_stride & 7) == 0;
+      const long long at = static_cast<long long>(row_base + qi) * p.out_stride + head * od;
+#pragma unroll 1
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32b_x32(o_addr + c * 32, o);
+        tmem_ld_wait();
+        if (!row_valid) continue;
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+          float f[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(o[i + e]) * inv;
+          const int col = c * 32 + i;
+          if (col >= od) continue;
+          if (vec && p.out_f32 != nullptr) {
+            float* d = p.out_f32 + at + col;
+            *reinterpret_cast<float4*>(d) = make_float4(f[0], f[1], f[2], f[3]);
+            *reinterpret_cast<float4*>(d + 4) = make_float4(f[4], f[5], f[6], f[7]);
+          } else if (vec) {
+            *reinterpret_cast<uint4*>(p.out + at + col) = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]),
+                                                                     pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              if (col + e >= od) continue;
+              if (p.out_f32 != nullptr) p.out_f32[at + col + e] = f[e];
+              else p.out[at + col + e] = __float2bfloat16(f[e]);
+            }
+          }
+        }
+      }
+    }
+    tc_fence_before_sync();
+  }
+
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+template <int D, bool EXACT>
+void launch_pair(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const PrefillAttnParams& p,
+                 int n_tiles, int* status, cudaStream_t stream) {
+  using L = PairSmem<D, EXACT>;
+  static_assert(L::kTotal <= 227 * 1024 && 256 + 2 * D <= 512, "tile budget");
+  auto kern = prefill_pair_kernel<D, EXACT>;
+  ensure_dynamic_smem(kern, L::kTotal);
+  kern<<<dim3(n_tiles, p.Hq / 2), kPairThreads, L::kTotal, stream>>>(tmQ, tmK, tmV, p, status);
+}
+
+}  // namespace
 
 void launch_paged_prefill_tc(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
                              const PrefillAttnParams& p, int n_tiles, int head_dim, int* status,
                              cudaStream_t stream) {
   if (n_tiles <= 0) return;
+  // a pair of heads must share its key head
+  if (p.Hq / p.Hkv % 2 == 0) {
+    if (head_dim == 128) {
+      if (p.exact_p != 0) launch_pair<128, true>(tmQ, tmK, tmV, p, n_tiles, status, stream);
+      else launch_pair<128, false>(tmQ, tmK, tmV, p, n_tiles, status, stream);
+    } else {
+      if (p.exact_p != 0) launch_pair<64, true>(tmQ, tmK, tmV, p, n_tiles, status, stream);
+      else launch_pair<64, false>(tmQ, tmK, tmV, p, n_tiles, status, stream);
+    }
+    return;
+  }
   if (head_dim == 128) {
     if (p.exact_p != 0) launch_tc<128, 128, 128, true>(tmQ, tmK, tmV, p, n_tiles, status, stream);
     else launch_tc<128, 128, 128, false>(tmQ, tmK, tmV, p, n_tiles, status, stream);

@@ -372,6 +372,10 @@ def test_paged_decode_block_mass(ops, hq, hkv, d, seq_lens, pps, window):
     (8, 1, 128, [(90, 300), (20, 20)], 48),
     (2, 1, 128, [(300, 700), (128, 128), (257, 257)], 0),
     (4, 2, 64, [(200, 500)], 100),
+    # pairs of heads: tiles that end at, before and behind a KV tile; three heads per key head go one by one
+    (4, 1, 128, [(127, 127), (128, 256), (129, 385), (1, 128), (1, 129)], 0),
+    (4, 2, 64, [(256, 1024), (2, 897)], 128),
+    (6, 2, 128, [(130, 260)], 0),
 ])
 def test_paged_prefill(ops, hq, hkv, d, chunks, window):
     torch.manual_seed(6)
