@@ -40,7 +40,7 @@
 // output projections (launch_wrappers.cu:202-247) and the host-loop grouped expert GEMM
 // (oxide-engine/src/moe_gemm.rs:208-345); the reference's all-reduce
 // (oxide-backend-cuda/src/nccl.rs:18-29) is a no-op.
-#include "gemm_bf16.cuh"
+#include "gemm_dev.cuh"
 #include "quant_expand.cuh"
 
 #include "../common/device_info.h"
@@ -73,11 +73,6 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
 __device__ __forceinline__ void red_relaxed_sys_add(uint32_t* p, uint32_t v) {
   asm volatile("red.relaxed.sys.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void red_add_v4_f32(float* p, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c),
-               "f"(d)
-               : "memory");
-}
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -85,29 +80,6 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 __device__ __forceinline__ void stamp(const GemmParams& p, int slot) {
   if (p.trace != nullptr) p.trace[static_cast<size_t>(blockIdx.x) * 8 + slot] = global_ns();
-}
-// SiLU / tanh-GELU on the special-function unit (approximate reciprocal and tanh: the result is
-// rounded to bf16 anyway); a full-precision divide and tanhf cost tens of instructions per value in
-// an epilogue that only one warp per scheduler runs.
-__device__ __forceinline__ float act_fn(float x, int act) {
-  if (act == 0) return __fdividef(x, 1.f + __expf(-x));
-  float t;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.7978845608028654f * (x + 0.044715f * x * x * x)));
-  return 0.5f * x * (1.f + t);
-}
-
-// NG groups of 32 accumulator columns of this thread's TMEM lane: all loads are issued before the
-// one wait (a load-wait pair costs a few hundred cycles).
-template <int NG>
-__device__ __forceinline__ void tmem_load_cols(uint32_t taddr, float (&a)[NG * 32]) {
-  uint32_t r[NG][32];
-#pragma unroll
-  for (int g = 0; g < NG; ++g) tmem_ld_32x32b_x32(taddr + g * 32, r[g]);
-  tmem_ld_wait();
-#pragma unroll
-  for (int g = 0; g < NG; ++g)
-#pragma unroll
-    for (int j = 0; j < 32; ++j) a[g * 32 + j] = __uint_as_float(r[g][j]);
 }
 // Waits until the source counters [s_lo, s_hi] reach the expected value; `waiters` is the number
 // of such waits the whole grid performs, the last of them re-arms the counters.
@@ -306,27 +278,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     int ok = 1;
     if (p.ag_flags != nullptr && lane == 0) ok = wait_sources(p, 0, p.ag_n_src - 1, gridDim.x) ? 1 : 0;
     ok = __shfl_sync(0xffffffffu, ok, 0);
-    int acc = 0;
-    for (int e0 = 0; e0 < p.n_groups; e0 += 32) {
-      const int e = e0 + lane;
-      const int rows = e >= p.n_groups ? 0 : (p.group_counts != nullptr ? static_cast<int>(__ldcg(p.group_counts + e)) : p.M);
-      const int tiles = (rows + BM - 1) / BM;
-      int incl = tiles;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += up;
-      }
-      if (e < p.n_groups) {
-        s_counts[e] = acc + incl - tiles;
-        s_rows[e] = rows;
-      }
-      acc += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) {
-      s_counts[p.n_groups] = acc;
-      s_misc[0] = ok;
-    }
+    group_tiles(p, BM, lane, s_counts, s_rows);
+    if (lane == 0) s_misc[0] = ok;
   }
   __syncthreads();  // barriers, start-up state
   // The producer warp goes ahead (its first weight tiles depend on no earlier kernel). The other

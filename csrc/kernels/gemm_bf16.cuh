@@ -108,6 +108,11 @@ int gemm_max_fixup_splits(int bn, int mt, bool swiglu);
 void launch_gemm_bf16(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int bn,
                       int mt, cudaStream_t stream);
 
+// The GEMM of CTA pairs (gemm_pair.cu): 256 x 256 tiles, maps with boxes of 128 rows. `gemm_pair_takes` says whether a
+// launch with these parameters has enough rows and tiles for it and asks for nothing that it does not do.
+bool gemm_pair_takes(const GemmParams& p, int mt);
+void launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream);
+
 // Activation quantiser of the NVFP4 GEMM: bf16 rows -> packed e2m1 + ue4m3 block scales (atom layout
 // above) + one fp32 scale per row (row amax / (448 * 6)). Rows are [groups, rows_per_group, K];
 // with group_counts only the first group_counts[g] rows of a group are converted. With wait.flags the

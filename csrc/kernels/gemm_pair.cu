@@ -1,0 +1,351 @@
+// tcgen05 bf16 GEMM of CTA pairs for steps with many rows (prompts): C[g][M, N] = A[g][M, K] * B[g][N, K]^T.
+//
+// A 128 x 256 tile of one CTA (gemm_bf16.cu) needs 48 KB of operands per 64 values of K while its MMAs take 512 clocks: 96 bytes
+// per clock through a port between L2 and an SM that moves 64, so the tensor core waits (1842 us, 0.62 of the measured cuBLAS rate, at
+// 8000 x 28672 x 4096). Here the two SMs of a TPC share a 256 x 256 tile (tcgen05 cta_group::2): each loads half of the rows of A and half
+// of the rows of B, 32 KB for the same 512 clocks, and both tensor cores read both halves of B: 1272 us
+// (1477 TFLOP/s; 1512 at 8192 x 8192 x 8192).
+//
+// Persistent, one pair per TPC; warp roles in each CTA: warp 0 = TMA producer, warp 1 = TMEM owner and, in the even CTA, MMA issuer
+// for both, warps 2..5 = epilogue of the CTA's own 128 rows. The operand ring has 6 stages; a stage is full when the bytes of both
+// CTAs have arrived at the even CTA's mbarrier, and empty when a commit that arrives at both CTAs says so. The accumulator is double
+// buffered in TMEM (2 x 256 columns). Tiles are walked in bands of kBand row tiles, so the tiles in flight (74 pairs) read
+// about 8 row tiles and 9 column tiles: 17 operand tiles per wave, against 74 + 1 in plain order.
+// Epilogues move 128 bytes per row and round through shared memory, so that stores and reductions are whole lines.
+// Every wait is bounded; a wait that runs out sets the status word, and all threads still meet at the cluster barrier of the end.
+#include "gemm_dev.cuh"
+
+#include "../common/device_info.h"
+
+namespace oxb {
+
+namespace {
+
+constexpr int kBK = 64;
+constexpr int kTile = 256;                     // rows and columns of a pair's tile
+constexpr int kHalf = 128;                     // rows of A and rows of B that one CTA holds
+constexpr int kOpBytes = kHalf * kBK * 2;      // one operand half of a stage
+constexpr int kStages = 6;
+constexpr int kBand = 8;
+constexpr int kPairThreads = 192;
+constexpr int kPitch = 144;                    // staged row: 128 bytes + 16 against bank conflicts
+constexpr int kStageOff = kStages * 2 * kOpBytes;
+constexpr int kBarOff = kStageOff + 128 * kPitch;
+constexpr int kSmem = kBarOff + 256 + 1024;
+constexpr uint32_t kCols = 512;
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kBarOff);   // [kStages], used in the even CTA
+  uint64_t* empty = full + kStages;                               // [kStages]
+  uint64_t* tmem_full = empty + kStages;                          // [2]
+  uint64_t* tmem_empty = tmem_full + 2;                           // [2], used in the even CTA
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  int* s_starts = reinterpret_cast<int*>(smem + kBarOff + 256);   // grouped: first tile of every group, then its rows
+  int* s_rows = s_starts + p.n_groups + 1;
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const uint32_t spin = spin_budget(p.spin_limit);
+  const int total_kb = (p.K + kBK - 1) / kBK;
+  const int n_tiles = (p.N + kTile - 1) / kTile;
+  const bool grouped = p.n_groups > 0;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tmem_full[b], 1);
+      mbar_init(&tmem_empty[b], 8);  // 4 epilogue warps of each CTA
+    }
+    fence_mbar_init();
+  }
+  pdl_wait();  // operands, counts and TMEM belong to earlier kernels until here
+  if (warp == 1) {
+    tmem_alloc_pair(tmem_slot, kCols);
+    tmem_relinquish_pair();
+  }
+  if (grouped && warp == 2) group_tiles(p, kTile, lane, s_starts, s_rows);
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();  // the other CTA's barriers are initialised
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  const int m_tiles = grouped ? s_starts[p.n_groups] : (p.M + kTile - 1) / kTile;
+  const int n_work = m_tiles * n_tiles;
+
+  struct Item {
+    int group, m0, rows, n0;
+  };
+  auto decode = [&](int w) -> Item {
+    const int band = w / (kBand * n_tiles);
+    const int left = m_tiles - band * kBand;
+    const int high = left < kBand ? left : kBand;
+    const int r = w - band * kBand * n_tiles;
+    int mt = band * kBand + r % high;
+    Item it;
+    it.n0 = r / high * kTile;
+    it.group = 0;
+    it.rows = p.M;
+    if (grouped) {
+      int lo = 0, hi = p.n_groups;  // the last group that starts at or before this tile
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (s_starts[mid] <= mt) lo = mid;
+        else hi = mid;
+      }
+      it.group = lo;
+      it.rows = s_rows[lo];
+      mt -= s_starts[lo];
+    }
+    it.m0 = mt * kTile + static_cast<int>(rank) * kHalf;
+    if (p.packed_rows) {  // groups one after the other, each from a multiple of 128 rows on
+      int first = 0;
+      for (int e = 0; e < it.group; ++e) first += (s_rows[e] + 127) / 128 * 128;
+      it.m0 += first;
+      it.rows += first;
+    }
+    return it;
+  };
+  const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
+
+  if (warp == 0) {
+    // ------------------------------ TMA producer ------------------------------
+    // lane = 2 * stage + operand: copies that one thread issues complete one after the other
+    uint32_t iter = 0;
+    bool ok = true;
+    for (int w = first; w < n_work && ok; w += step) {
+      const Item it = decode(w);
+      const int b_row = it.n0 + static_cast<int>(rank) * kHalf;
+      for (int kb = 0; kb < total_kb; ++kb, ++iter) {
+        const int s = iter % kStages;
+        if (iter >= kStages && !mbar_wait(&empty[s], (iter / kStages - 1) & 1, spin)) ok = false;
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutProducer);
+          break;
+        }
+        if (rank == 0 && lane == 0) mbar_arrive_expect_tx(&full[s], 4 * kOpBytes);
+        __syncwarp();
+        uint8_t* stage = smem + s * 2 * kOpBytes;
+        const int op = lane - 2 * s;
+        if (op == 0) {
+          tma_load_3d_pair(stage, &tmA, cluster_addr(&full[s], 0), kb * kBK, it.m0, p.packed_rows ? 0 : it.group);
+        } else if (op == 1) {
+          if (p.b_tiled)
+            tma_load_3d_pair(stage + kOpBytes, &tmB, cluster_addr(&full[s], 0), 0, 0, (b_row >> 7) * total_kb + kb);
+          else
+            tma_load_3d_pair(stage + kOpBytes, &tmB, cluster_addr(&full[s], 0), kb * kBK, b_row, it.group);
+        }
+      }
+    }
+    if (lane == 0) pdl_launch_dependents();  // every operand of this CTA has been requested
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer (even CTA) ---------------------
+    if (rank == 0 && lane == 0) {
+      constexpr uint32_t idesc = make_idesc(kFmtBF16, kFmtBF16, kTile, kTile);
+      uint32_t iter = 0, t = 0;
+      bool ok = true;
+      for (int w = first; w < n_work && ok; w += step, ++t) {
+        const uint32_t buf = t & 1, use = t >> 1;
+        if (use >= 1 && !mbar_wait_cluster(&tmem_empty[buf], (use & 1) ^ 1, spin)) ok = false;
+        tc_fence_after_sync();
+        for (int kb = 0; kb < total_kb && ok; ++kb, ++iter) {
+          const int s = iter % kStages;
+          if (!mbar_wait_cluster(&full[s], (iter / kStages) & 1, spin)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t a = smem_u32(smem + s * 2 * kOpBytes), b = a + kOpBytes;
+#pragma unroll
+          for (int k = 0; k < kBK / 16; ++k)
+            tc_mma_f16_pair(tmem_base + buf * kTile, make_desc_kmajor_sw128(a + k * 32), make_desc_kmajor_sw128(b + k * 32),
+                            idesc, (kb | k) != 0 ? 1u : 0u);
+          tc_commit_pair(&empty[s]);
+        }
+        if (ok) tc_commit_pair(&tmem_full[buf]);
+      }
+      if (!ok) set_status_once(p.status, kStatusMbarTimeoutMma);
+    }
+  } else {
+    // ------------------------------ epilogue ----------------------------------
+    const int q = warp & 3;  // TMEM lane quarter of this warp
+    uint8_t* stage = smem + kStageOff + q * 32 * kPitch;
+    uint8_t* my_row = stage + lane * kPitch;
+    const bool swiglu = p.epi == kEpiSwigluBf16;
+    const bool wide_out = p.epi == kEpiRedF32 || p.epi == kEpiStoreF32;  // fp32 rows: 32 columns per round, else 64
+    const int n_out = swiglu ? p.N >> 1 : p.N;
+    uint32_t t = 0;
+    for (int w = first; w < n_work; w += step, ++t) {
+      const Item it = decode(w);
+      const uint32_t buf = t & 1;
+      bool ok = mbar_wait(&tmem_full[buf], (t >> 1) & 1, spin);
+      ok = __all_sync(0xffffffffu, ok);  // tcgen05.ld below is warp-collective
+      if (!ok) {
+        if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutEpilogue);
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t acc = tmem_base + buf * kTile + (static_cast<uint32_t>(q * 32) << 16);
+      const int row0 = it.m0 + q * 32;  // first row of this warp
+      const __nv_bfloat16* bias = p.bias != nullptr ? p.bias + static_cast<long long>(it.group) * p.N : nullptr;
+      // where this lane's row goes in a routed sum
+      int dst_row = row0 + lane;
+      float wgt = 1.f;
+      if (p.row_meta != nullptr && row0 + lane < it.rows) {
+        const RowMeta m = p.row_meta[it.group * p.meta_group_stride + row0 + lane];
+        dst_row = m.row;
+        wgt = m.weight;
+      }
+      // 16 bytes of a staged row to their place: 8 lanes per row, 4 rows per instruction
+      auto copy_out = [&](int col) {  // col: first output column of the round
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rr = i * 4 + (lane >> 3);
+          const int row = row0 + rr;
+          const uint4 x = *reinterpret_cast<const uint4*>(stage + rr * kPitch + (lane & 7) * 16);
+          const int to = __shfl_sync(0xffffffffu, dst_row, rr);
+          const int c = col + (lane & 7) * (wide_out ? 4 : 8);
+          if (row >= it.rows || c >= n_out) continue;
+          if (p.epi == kEpiRedF32) {
+            float* d = p.dst[0] + static_cast<long long>(to) * p.dst_ld + c;
+            if ((p.dst_ld & 3) == 0 && c + 4 <= n_out) {
+              red_add_v4_f32(d, __uint_as_float(x.x), __uint_as_float(x.y), __uint_as_float(x.z), __uint_as_float(x.w));
+            } else {
+              const float f[4] = {__uint_as_float(x.x), __uint_as_float(x.y), __uint_as_float(x.z), __uint_as_float(x.w)};
+              for (int e = 0; e < 4 && c + e < n_out; ++e) atomicAdd(d + e, f[e]);
+            }
+          } else if (p.epi == kEpiStoreF32) {
+            float* d = reinterpret_cast<float*>(p.C) + static_cast<long long>(it.group) * p.c_group_stride +
+                       static_cast<long long>(row) * p.ldc + c;
+            if ((p.ldc & 3) == 0 && (p.c_group_stride & 3) == 0 && c + 4 <= n_out) {
+              *reinterpret_cast<uint4*>(d) = x;
+            } else {
+              const float f[4] = {__uint_as_float(x.x), __uint_as_float(x.y), __uint_as_float(x.z), __uint_as_float(x.w)};
+              for (int e = 0; e < 4 && c + e < n_out; ++e) d[e] = f[e];
+            }
+          } else {
+            __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<long long>(it.group) * p.c_group_stride +
+                               static_cast<long long>(row) * p.ldc + c;
+            if ((p.ldc & 7) == 0 && (p.c_group_stride & 7) == 0 && c + 8 <= n_out) {
+              *reinterpret_cast<uint4*>(d) = x;
+            } else {
+              const __nv_bfloat16* e8 = reinterpret_cast<const __nv_bfloat16*>(&x);
+              for (int e = 0; e < 8 && c + e < n_out; ++e) d[e] = e8[e];
+            }
+          }
+        }
+        __syncwarp();
+      };
+#pragma unroll 1
+      for (int c = 0; c < kTile; c += 64) {
+        if (it.n0 + c >= p.N) break;
+        float a[64];
+        tmem_load_cols<2>(acc + c, a);
+        if (swiglu) {  // 32 gate | 32 up: 32 outputs, half of a staged row
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = act_fn(a[j + e], p.act) * a[32 + j + e];
+            *reinterpret_cast<uint4*>(my_row + ((c & 64) >> 1) * 2 + j * 2) =
+                make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+          }
+          if (c & 64) copy_out(((it.n0 + c) >> 1) - 32);
+          continue;
+        }
+        if (bias != nullptr && p.epi != kEpiRedF32) {
+#pragma unroll
+          for (int j = 0; j < 64; ++j)
+            if (it.n0 + c + j < p.N) a[j] += __bfloat162float(bias[it.n0 + c + j]);
+        }
+        if (wide_out) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+              *reinterpret_cast<float4*>(my_row + j * 4) =
+                  make_float4(wgt * a[h * 32 + j], wgt * a[h * 32 + j + 1], wgt * a[h * 32 + j + 2], wgt * a[h * 32 + j + 3]);
+            copy_out(it.n0 + c + h * 32);
+          }
+          continue;
+        }
+        if (p.act == 2) {
+#pragma unroll
+          for (int j = 0; j < 64; ++j) {
+            const float r = fmaxf(a[j], 0.f);
+            a[j] = r * r;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 64; j += 8)
+          *reinterpret_cast<uint4*>(my_row + j * 2) = make_uint4(pack_bf16x2(a[j], a[j + 1]), pack_bf16x2(a[j + 2], a[j + 3]),
+                                                                 pack_bf16x2(a[j + 4], a[j + 5]), pack_bf16x2(a[j + 6], a[j + 7]));
+        copy_out(it.n0 + c);
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(cluster_addr(&tmem_empty[buf], 0));
+    }
+    if (p.done_ticket != nullptr) {
+      // the last CTA of the grid re-arms the caller's words (one GPU: nothing to signal)
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (warp == 2 && lane == 0) {
+        __threadfence();
+        if (atomicAdd(p.done_ticket, 1u) == gridDim.x - 1) {
+          for (int i = 0; i < p.n_reset; ++i) p.reset_on_done[i] = 0;
+          *p.done_ticket = 0;
+        }
+      }
+    }
+    tc_fence_before_sync();
+  }
+
+  __syncthreads();
+  cluster_sync_all();  // no CTA leaves while the other may still signal it or work in its memory
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc_pair(tmem_base, kCols);
+  }
+}
+
+}  // namespace
+
+bool gemm_pair_takes(const GemmParams& p, int mt) {
+  // one GPU's own rows, whole K: what needs flags, peers, splits or other operands stays with gemm_bf16.cu
+  if (p.kind != 0 || mt != 1 || p.splits != 1 || p.ag_flags != nullptr || p.trace != nullptr || p.epi == kEpiSlabBf16) return false;
+  if (p.epi == kEpiRedF32) {
+    if (p.n_owners != 1 || (p.row_meta == nullptr && p.rows_per_owner < p.M)) return false;
+    for (int o = 0; o < kMaxRanks; ++o)
+      if (p.arrive[o] != nullptr) return false;
+  }
+  if (p.epi == kEpiSwigluBf16 && p.N % kTile != 0) return false;
+  const int n_tiles = (p.N + kTile - 1) / kTile;
+  const int pairs = sm_count() / 2;
+  if (p.n_groups > 0 && p.group_counts == nullptr) return p.M >= kTile && p.n_groups * ((p.M + kTile - 1) / kTile) * n_tiles >= pairs;
+  // grouped: m_tiles bounds the 128-row tiles of all groups, one unfinished tile per group included
+  if (p.n_groups > 0) return p.m_tiles - p.n_groups >= 2 * p.n_groups && (p.m_tiles - p.n_groups) / 2 * n_tiles >= pairs;
+  return p.M > kTile && (p.M + kTile - 1) / kTile * n_tiles >= pairs;
+}
+
+void launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
+  const size_t smem = kSmem + (p.n_groups > 0 ? (2 * static_cast<size_t>(p.n_groups) + 1) * sizeof(int) : 0);
+  ensure_dynamic_smem(gemm_pair_kernel, smem);
+  const int n_tiles = (p.N + kTile - 1) / kTile;
+  const int m_tiles = p.n_groups > 0 ? p.m_tiles : (p.M + kTile - 1) / kTile;
+  const int pairs = sm_count() / 2;
+  const int n_work = m_tiles * n_tiles;
+  launch_kernel(gemm_pair_kernel, dim3(2 * (n_work < pairs ? n_work : pairs)), dim3(kPairThreads), smem, stream,
+                /*pdl=*/true, /*cooperative=*/false, tmA, tmB, p);
+}
+
+}  // namespace oxb

@@ -249,6 +249,81 @@ def test_gemm_grouped_combine(ops):
     assert cnt_copy.abs().max().item() == 0 and ticket.item() == 0
 
 
+@pytest.mark.parametrize("m,n,k,tiled", [
+    (257, 9600, 136, False), (2049, 3000, 72, False), (513, 6400, 256, True), (1100, 3968, 1024, True), (4100, 1160, 64, False),
+])
+def test_gemm_of_cta_pairs(ops, m, n, k, tiled):
+    """Sizes of the 256 x 256 tiles: a row beyond a tile, ragged columns and depths, more tiles than pairs, every epilogue."""
+    torch.manual_seed(m)
+    a = torch.randn(m, k, device=DEV, dtype=torch.bfloat16)
+    w = torch.randn(n, k, device=DEV, dtype=torch.bfloat16)
+    b = torch.randn(n, device=DEV, dtype=torch.bfloat16)
+    wt = ops.tile_weight(w) if tiled else w
+    assert tiled == (wt.dim() == 4)
+    ref = a.double() @ w.double().T
+    bf16 = 2.0 ** -8   # half an ulp of the results, which are a row's largest value or less
+    assert _rel_err(ops.gemm(a, wt, bn=256), ref) < bf16
+    assert _rel_err(ops.gemm(a, wt, bias=b, act=2, bn=128), (ref + b.double()).clamp_min(0).square()) < 2 * bf16
+    out = torch.full((m, n + 8), 7.0, device=DEV)
+    ops.gemm(a, wt, out=out[:, :n], epi=ops.EPI_STORE_F32, bias=b, bn=128)
+    assert _rel_err(out[:, :n], ref + b.double()) < 1e-5 and (out[:, n:] == 7.0).all()
+    acc = torch.ones(m, n, device=DEV)
+    ops.gemm(a, wt, epi=ops.EPI_RED_F32, dst_ptrs=[acc.data_ptr()], bn=128)
+    assert _rel_err(acc, ref + 1) < 1e-5
+    if n % 256 == 0:
+        gu = ops.gemm(a, wt, epi=ops.EPI_SWIGLU_BF16, bn=256)
+        v = ref.view(m, n // 64, 2, 32)
+        assert _rel_err(gu, (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(m, n // 2)) < 2 * bf16
+    torch.cuda.synchronize()
+    ops.check_status()
+
+
+def test_grouped_gemm_of_cta_pairs(ops):
+    """Groups with uneven and no rows in slabs, packed one after the other, and of equal size; the weighted sum of the routed form."""
+    torch.manual_seed(5)
+    G, cap, k, n = 5, 1100, 192, 6400
+    counts = torch.tensor([700, 0, 1, 1100, 257], dtype=torch.int32, device=DEV)
+    a = torch.randn(G, cap, k, device=DEV, dtype=torch.bfloat16)
+    w = torch.randn(G, n, k, device=DEV, dtype=torch.bfloat16)
+    m_tiles = 2058 // 128 + G
+    ref = torch.einsum("gmk,gnk->gmn", a.double(), w.double())
+    out = torch.zeros(G, cap, n, device=DEV, dtype=torch.bfloat16)
+    ops.gemm(a, w, out=out, group_counts=counts, m_tiles=m_tiles, bn=128)
+    for g, c in enumerate(counts.tolist()):
+        assert c == 0 or _rel_err(out[g, :c], ref[g, :c]) < 2.0 ** -8
+        assert (out[g, c:] == 0).all()
+    T = 900
+    meta = torch.zeros(G, cap, 4, dtype=torch.int32, device=DEV)
+    rows, wts = torch.randint(0, T, (G, cap), device=DEV, dtype=torch.int32), torch.rand(G, cap, device=DEV)
+    meta[:, :, 1], meta[:, :, 2] = rows, wts.view(torch.int32)
+    acc = torch.zeros(T, n, device=DEV)
+    ticket, left = torch.zeros(1, dtype=torch.int32, device=DEV), counts.clone()
+    ops.gemm(a, w, epi=ops.EPI_RED_F32, dst_ptrs=[acc.data_ptr()], group_counts=left, row_meta=meta, m_tiles=m_tiles, bn=128,
+             done_ticket=ticket, reset_on_done=left)
+    want = torch.zeros(T, n, device=DEV, dtype=torch.float64)
+    for g, c in enumerate(counts.tolist()):
+        want.index_add_(0, rows[g, :c].long(), ref[g, :c] * wts[g, :c, None].double())
+    assert _rel_err(acc, want) < 1e-5 and int(left.abs().max()) == 0 and int(ticket) == 0
+    # packed: every group from a multiple of 128 rows on
+    starts, at = [], 0
+    for c in counts.tolist():
+        starts.append(at)
+        at += (c + 127) // 128 * 128
+    rows_total = at + 256
+    pa = torch.randn(rows_total, k, device=DEV, dtype=torch.bfloat16)
+    po = torch.zeros(rows_total, n, device=DEV, dtype=torch.bfloat16)
+    ops.gemm(pa, w, out=po, group_counts=counts, m_tiles=rows_total // 128, bn=128)
+    for g, c in enumerate(counts.tolist()):
+        if c:
+            assert _rel_err(po[starts[g]:starts[g] + c], pa[starts[g]:starts[g] + c].double() @ w[g].double().T) < 2.0 ** -8
+        end = starts[g + 1] if g + 1 < G else at
+        assert (po[starts[g] + c:end] == 0).all()
+    eq = ops.gemm(a[:, :600], w, out=torch.empty(G, 600, n, device=DEV, dtype=torch.bfloat16), bn=128)
+    assert _rel_err(eq, ref[:, :600]) < 2.0 ** -8
+    torch.cuda.synchronize()
+    ops.check_status()
+
+
 # ------------------------------------------------------------------------------------- attention
 def _make_paged(seq_lens, hkv, d, extra_blocks=3, seed=0):
     g = torch.Generator(device="cpu").manual_seed(seed)
