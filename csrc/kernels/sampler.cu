@@ -1,25 +1,35 @@
 // Device sampler (sm_100a): per-row greedy argmax, and temperature / top-k / min-p / top-p
 // sampling with an optional allow-bitmask (grammar, banned tokens).
 //
-// One CTA per row. Sampling path: 4-pass radix select of the C = max(top_k, 256) largest
-// logits (C <= 1024) -> gather -> bitonic sort in shared memory -> softmax over the candidates
-// -> min-p -> top-k -> top-p -> renormalise -> inverse-CDF draw from a counter-based RNG.
+// Sampling takes the C = max(top_k, 256) largest logits (C <= 1024), sorts them, and then: softmax over the
+// candidates -> min-p -> top-k -> top-p -> renormalise -> inverse-CDF draw from a counter-based RNG.
 // The order of the filters is the reference's (oxide-core/src/sampler.rs:173-390, which
 // also truncates to max(k,256) candidates before the softmax, sampler.rs:274-280).
 // Replaces argmax_f32_kernel / argmax_stage1/2 (sampling_dfa.cu:2-159) and the Gumbel-max
 // sample_stage1 kernel (sampling_dfa.cu:180-274), whose top_p argument is ignored.
 #include "sampler.cuh"
 
+#include <cooperative_groups.h>
 #include <math.h>
 
+#include <type_traits>
+
+#include "../common/device_info.h"
 #include "../common/sm100.cuh"
 
 namespace oxb {
 
 namespace {
 
-constexpr int kThreads = 1024;
-constexpr int kMaxCand = 1024;
+namespace cg = cooperative_groups;
+
+constexpr int kThreads = 1024;       // argmax kernels
+constexpr int kMaxCand = 1024;       // candidates that the filters see at most
+constexpr int kSampleThreads = 512;
+constexpr int kSampleCap = 2048;     // candidates that the threshold may let through
+constexpr int kBins = 2048;          // 11 bits of a key, then
+constexpr int kBins2 = 1024;         // ten more
+constexpr int kMaxSlices = 8;
 
 __device__ __forceinline__ uint32_t f2key(float f) {
   uint32_t u = __float_as_uint(f);
@@ -35,19 +45,10 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
   return x ^ (x >> 31);
 }
 
-__device__ void block_argmax(const float* row, const uint32_t* mask, int V, int* out_idx,
-                             float* out_val) {
+// (value, index) of every thread -> the largest value of the CTA and the lowest index that has it (0x7fffffff: none).
+__device__ void reduce_argmax(float best, int bi, int* out_idx, float* out_val) {
   __shared__ float s_v[32];
   __shared__ int s_i[32];
-  float best = -INFINITY;
-  int bi = 0x7fffffff;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float v = allowed(mask, i) ? row[i] : -INFINITY;
-    if (v > best || (v == best && i < bi)) {
-      best = v;
-      bi = i;
-    }
-  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -77,49 +78,45 @@ __device__ void block_argmax(const float* row, const uint32_t* mask, int V, int*
       }
     }
     if (lane == 0) {
-      *out_idx = bi == 0x7fffffff ? 0 : bi;
+      *out_idx = bi;
       *out_val = best;
     }
   }
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads) sample_kernel(const SampleParams p) {
-  __shared__ int s_hist[256];
-  __shared__ float s_val[kMaxCand];
-  __shared__ int s_idx[kMaxCand];
-  __shared__ int s_count, s_tok;
-  __shared__ uint32_t s_prefix;
-  __shared__ int s_remaining;
-  __shared__ float s_best;
-
-  const int row = blockIdx.x;
-  const float* logits = p.logits + static_cast<long long>(row) * p.ld;
-  const uint32_t* mask =
-      p.allow_mask != nullptr ? p.allow_mask + static_cast<long long>(row) * p.mask_words : nullptr;
-  const int V = p.V;
-  const float temp = p.temperature != nullptr ? p.temperature[row] : 0.f;
-  int top_k = p.top_k != nullptr ? p.top_k[row] : 0;
-  const float top_p = p.top_p != nullptr ? p.top_p[row] : 1.f;
-  const float min_p = p.min_p != nullptr ? p.min_p[row] : 0.f;
-
-  if (temp <= 0.f || top_k == 1) {
-    block_argmax(logits, mask, V, &s_tok, &s_best);
-    if (threadIdx.x == 0) {
-      p.out_tokens[row] = s_tok;
-      if (p.out_logit != nullptr) p.out_logit[row] = s_best;
+__device__ void block_argmax(const float* row, int V, int* out_idx, float* out_val) {
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  for (int i = threadIdx.x; i < V; i += blockDim.x) {
+    const float v = row[i];
+    if (v > best || (v == best && i < bi)) {
+      best = v;
+      bi = i;
     }
-    return;
   }
-  if (top_k <= 0 || top_k > V) top_k = V;
-  int C = top_k > 256 ? top_k : 256;
-  if (C > kMaxCand) C = kMaxCand;
-  if (C > V) C = V;
+  reduce_argmax(best, bi, out_idx, out_val);
+  if (threadIdx.x == 0 && *out_idx == 0x7fffffff) *out_idx = 0;
+  __syncthreads();
+}
 
-  // ---- radix select: key of the C-th largest allowed logit ----
+__device__ __forceinline__ float key2f(uint32_t k) {
+  return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
+}
+// Sort word of a candidate: larger value first, then the lower index (both zeros are one value).
+__device__ __forceinline__ unsigned long long cand_word(float v, int i) {
+  return (static_cast<unsigned long long>(f2key(v + 0.f)) << 32) | (0xFFFFFFFFu - static_cast<uint32_t>(i));
+}
+
+// Exact radix select of the C largest allowed logits by one CTA, for rows where too many logits share the threshold of
+// sample_kernel (thousands of equal ones). Returns the number of words in `out`.
+__device__ int select_exact(const float* logits, const uint32_t* mask, int V, int C, int* s_hist, unsigned long long* out) {
+  __shared__ uint32_t s_prefix;
+  __shared__ int s_left, s_n;
   if (threadIdx.x == 0) {
     s_prefix = 0;
-    s_remaining = C;
+    s_left = C;
+    s_n = 0;
   }
   __syncthreads();
   for (int pass = 0; pass < 4; ++pass) {
@@ -135,150 +132,452 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const SampleParams p) 
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      int rem = s_remaining;
+      int rem = s_left;
       int b = 255;
       for (; b > 0; --b) {
         if (s_hist[b] >= rem) break;
         rem -= s_hist[b];
       }
       s_prefix = prefix | (static_cast<uint32_t>(b) << shift);
-      s_remaining = rem;
+      s_left = rem;
     }
     __syncthreads();
   }
   const uint32_t kth = s_prefix;
-
-  // ---- gather candidates: everything above the threshold, ties until C is reached ----
-  if (threadIdx.x == 0) s_count = 0;
-  for (int i = threadIdx.x; i < kMaxCand; i += blockDim.x) {
-    s_val[i] = -INFINITY;
-    s_idx[i] = 0x7fffffff;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    if (!allowed(mask, i)) continue;
-    const float v = logits[i];
-    if (f2key(v) > kth) {
-      const int s = atomicAdd(&s_count, 1);
-      if (s < kMaxCand) {
-        s_val[s] = v;
-        s_idx[s] = i;
+  // everything above the threshold (fewer than C), then ties until C is reached
+  for (int eq = 0; eq < 2; ++eq) {
+    for (int i = threadIdx.x; i < V; i += blockDim.x) {
+      if (!allowed(mask, i)) continue;
+      const float v = logits[i];
+      const uint32_t k = f2key(v);
+      if (eq ? k == kth : k > kth) {
+        const int s = atomicAdd(&s_n, 1);
+        if (s < C) out[s] = cand_word(v, i);
       }
     }
+    __syncthreads();
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    if (!allowed(mask, i)) continue;
-    const float v = logits[i];
-    if (f2key(v) == kth) {
-      const int s = atomicAdd(&s_count, 1);
-      if (s < C) {
-        s_val[s] = v;
-        s_idx[s] = i;
-      }
-    }
-  }
-  __syncthreads();
-  int n = s_count < C ? s_count : C;
+  const int n = s_n;
+  return n < C ? n : C;
+}
 
-  // ---- bitonic sort, descending by value then ascending by index (deterministic) ----
-  for (int k = 2; k <= kMaxCand; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      const int i = threadIdx.x;
-      const int ixj = i ^ j;
-      if (ixj > i) {
-        const float a = s_val[i], b = s_val[ixj];
-        const int ia = s_idx[i], ib = s_idx[ixj];
-        const bool a_first = a > b || (a == b && ia < ib);  // a sorts before b
-        const bool up = (i & k) == 0;
-        if (up ? !a_first : a_first) {
-          s_val[i] = b;
-          s_val[ixj] = a;
-          s_idx[i] = ib;
-          s_idx[ixj] = ia;
+__device__ __forceinline__ float max_nan(float a, float b) {  // a NaN stays one
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+// One cluster of CTAs per row; each CTA reads its slice of the row once.
+//  1. Every thread keeps the maximum of four interleaved groups of its slice (and, with top-k off, its part of the softmax denominator). The C-th
+//     largest of all group maxima (two histogram passes over them, summed across the cluster) is no larger than the C-th largest
+//     logit, and few logits beyond the C largest reach it, since large ones rarely share a group: 2048 groups per CTA let
+//     through 1.0 to 1.4 C.
+//  2. The threads whose maximum reaches it read their groups again and send what does to the cluster's first CTA.
+//  3. That one sorts the candidates, takes the C largest, and filters and draws with block-wide scans.
+// What bounds it at 64 rows of 128256 (33 MB, 27 us; 239 us for one CTA per row with a radix select over the row, whose seven passes
+// met in a few bins of their histogram, and a serial tail): the read takes 7 us, the two thresholds with their cluster barriers
+// 8 to 10, gathering 5, the sort 4.
+__global__ void __launch_bounds__(kSampleThreads, 2) sample_kernel(const SampleParams p) {
+  __shared__ __align__(16) int s_hist[kBins];
+  __shared__ __align__(16) unsigned long long s_cand[kSampleCap];
+  __shared__ __align__(16) unsigned long long s_sort[kSampleCap];  // of the whole row, in the cluster's first CTA
+  __shared__ __align__(16) int s_hist2[kBins2];
+  __shared__ int s_scan[kSampleThreads / 32];
+  __shared__ float s_fscan[kSampleThreads / 32], s_fmax[kSampleThreads / 32];
+  __shared__ uint32_t s_bin;
+  __shared__ int s_above, s_count, s_total, s_base, s_tok, s_first;
+  __shared__ float s_best, s_part[kMaxSlices], s_part_max[kMaxSlices], s_tot;
+
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int S = static_cast<int>(cluster.num_blocks());
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int row = blockIdx.x / S;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float* logits = p.logits + static_cast<long long>(row) * p.ld;
+  const uint32_t* mask =
+      p.allow_mask != nullptr ? p.allow_mask + static_cast<long long>(row) * p.mask_words : nullptr;
+  const int V = p.V;
+  const float temp = p.temperature != nullptr ? p.temperature[row] : 0.f;
+  int top_k = p.top_k != nullptr ? p.top_k[row] : 0;
+  const float top_p = p.top_p != nullptr ? p.top_p[row] : 1.f;
+  const float min_p = p.min_p != nullptr ? p.min_p[row] : 0.f;
+  // this CTA's slice, in groups of four logits
+  const int per = ((V + 3) / 4 + S - 1) / S;
+  const int v_lo = rank * per;
+  const int v_hi = v_lo + per < (V + 3) / 4 ? v_lo + per : (V + 3) / 4;
+  const bool vec = (reinterpret_cast<uintptr_t>(logits) & 15) == 0;
+  // vectors [v_lo, v_fast) are whole, aligned and unmasked, [v_fast, v_hi) anything
+  const int v_fast = !vec || mask != nullptr ? v_lo : (v_hi < V / 4 ? v_hi : (V / 4 > v_lo ? V / 4 : v_lo));
+  // four logits from 4 v on; ok: bit e set where logit 4 v + e exists and is allowed
+  auto load4 = [&](int v, float (&x)[4], uint32_t& ok) __attribute__((always_inline)) {
+    const int i = 4 * v;
+    ok = i + 4 <= V ? 15u : (1u << (V - i)) - 1u;
+    if (vec && ok == 15u) {
+      const float4 q = __ldcg(reinterpret_cast<const float4*>(logits + i));
+      x[0] = q.x, x[1] = q.y, x[2] = q.z, x[3] = q.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] = (ok >> e) & 1u ? __ldcg(logits + i + e) : 0.f;
+    }
+    if (mask != nullptr) ok &= mask[i >> 5] >> (i & 31);
+  };
+
+  if (temp <= 0.f || top_k == 1) {
+    // greedy: the largest allowed logit, the lowest index among equal ones
+    float best = -INFINITY;
+    int bi = 0x7fffffff;
+    for (int v = v_lo + tid; v < v_hi; v += kSampleThreads) {
+      float x[4];
+      uint32_t ok;
+      load4(v, x, ok);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float y = (ok >> e) & 1u ? x[e] : -INFINITY;
+        const int i = 4 * v + e;
+        if (i < V && (y > best || (y == best && i < bi))) {
+          best = y;
+          bi = i;
         }
       }
-      __syncthreads();
     }
+    reduce_argmax(best, bi, &s_tok, &s_best);
+    cluster.sync();
+    if (rank == 0 && tid == 0) {
+      for (int r = 1; r < S; ++r) {  // slices in order: a later one wins only with a larger value
+        const float v = *cluster.map_shared_rank(&s_best, r);
+        if (v > s_best || (s_tok == 0x7fffffff && v == s_best)) {
+          s_best = v;
+          s_tok = *cluster.map_shared_rank(&s_tok, r);
+        }
+      }
+      p.out_tokens[row] = s_tok == 0x7fffffff ? 0 : s_tok;
+      if (p.out_logit != nullptr) p.out_logit[row] = s_best;
+    }
+    cluster.sync();  // shared memory that a peer reads stays until here
+    return;
   }
+  if (top_k <= 0 || top_k > V) top_k = V;
+  int C = top_k > 256 ? top_k : 256;
+  if (C > kMaxCand) C = kMaxCand;
+  if (C > V) C = V;
 
-  // ---- with top-k off the candidates are only the 1024 largest logits: the softmax denominator
-  // (what top-p and the reported log-probability are measured against) is taken over every allowed
-  // logit, so the thresholds are those of the full distribution ----
+  // ---- 1. maxima of the groups (key 0: empty), threshold ----
+  for (int i = tid; i < kBins; i += kSampleThreads) s_hist[i] = 0;
+  for (int i = tid; i < kBins2; i += kSampleThreads) s_hist2[i] = 0;
+  if (tid == 0) {
+    s_count = s_total = 0;
+  }
+  // with top-k off the candidates are only the 1024 largest logits, and the softmax denominator (what top-p and the reported
+  // log-probability are measured against) is taken over every allowed logit: the thresholds are those of the full distribution
   const bool full_mass = top_k >= V && V > C;
-  if (full_mass && n > 0) {
-    const float inv_t = 1.f / temp;
-    const float mx = s_val[0] * inv_t;
-    float part = 0.f;
-    for (int i = threadIdx.x; i < V; i += blockDim.x)
-      if (allowed(mask, i)) part += __expf(logits[i] * inv_t - mx);
+  const float inv_t = 1.f / temp;
+  constexpr int kBatch = 8;  // loads in flight per thread
+  float gmax[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  float run_m = -INFINITY, run_s = 0.f;  // largest logit so far, sum of exponentials relative to it
+  auto take = [&](const float4 (&x)[kBatch]) __attribute__((always_inline)) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    float* s_part = reinterpret_cast<float*>(s_hist);
-    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = part;
+    for (int u = 0; u < kBatch; ++u) {
+      gmax[0] = max_nan(gmax[0], x[u].x);
+      gmax[1] = max_nan(gmax[1], x[u].y);
+      gmax[2] = max_nan(gmax[2], x[u].z);
+      gmax[3] = max_nan(gmax[3], x[u].w);
+    }
+    if (!full_mass) return;
+    const float m = max_nan(max_nan(gmax[0], gmax[1]), max_nan(gmax[2], gmax[3]));
+    const float sub = m == -INFINITY ? 0.f : m * inv_t;
+    run_s *= __expf(run_m * inv_t - sub);
+    run_m = m;
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u)
+      run_s += (__expf(x[u].x * inv_t - sub) + __expf(x[u].y * inv_t - sub)) + (__expf(x[u].z * inv_t - sub) + __expf(x[u].w * inv_t - sub));
+  };
+  const float4 none = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+  for (int v = v_lo + tid; v < v_fast; v += kBatch * kSampleThreads) {
+    float4 x[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u)
+      x[u] = v + u * kSampleThreads < v_fast ? __ldcg(reinterpret_cast<const float4*>(logits) + v + u * kSampleThreads) : none;
+    take(x);
+  }
+  for (int v = v_fast + tid; v < v_hi; v += kBatch * kSampleThreads) {
+    float4 x[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      x[u] = none;
+      float y[4];
+      uint32_t ok;
+      if (v + u * kSampleThreads >= v_hi) continue;
+      load4(v + u * kSampleThreads, y, ok);
+      x[u] = make_float4(ok & 1u ? y[0] : -INFINITY, ok & 2u ? y[1] : -INFINITY, ok & 4u ? y[2] : -INFINITY, ok & 8u ? y[3] : -INFINITY);
+    }
+    take(x);
+  }
+  uint32_t gm[4];  // keys of the maxima; 0: nothing above minus infinity
+#pragma unroll
+  for (int e = 0; e < 4; ++e) gm[e] = gmax[e] == -INFINITY ? 0u : f2key(gmax[e]);
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (gm[e] != 0) atomicAdd(&s_hist[gm[e] >> 21], 1);
+  // The bin of the cluster's histogram `h` in which the `want`-th largest key lies; s_above = keys above that bin. False: there are
+  // fewer keys. PER bins per thread, the threads in descending order.
+  auto find_bin = [&](auto per_thread, int* h, int want) -> bool {
+    constexpr int PER = decltype(per_thread)::value;
+    const int first = PER * (kSampleThreads - 1 - tid);
+    cluster.sync();
+    int q[kMaxSlices][PER];
+#pragma unroll
+    for (int r = 0; r < kMaxSlices; ++r) {  // all remote loads in flight together
+      const int* from = cluster.map_shared_rank(h, r < S ? r : 0) + first;
+#pragma unroll
+      for (int i = 0; i < PER; i += 2) {
+        const int2 x = r < S ? *reinterpret_cast<const int2*>(from + i) : make_int2(0, 0);
+        q[r][i] = x.x;
+        q[r][i + 1] = x.y;
+      }
+    }
+    int mine = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+#pragma unroll
+      for (int r = 1; r < kMaxSlices; ++r) q[0][i] += q[r][i];
+      mine += q[0][i];
+    }
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += x;
+    }
+    if (lane == 31) s_scan[warp] = upto;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      float t = 0.f;
-      for (int w = 0; w < (blockDim.x >> 5); ++w) t += s_part[w];
-      s_best = t;
+    int total = 0;
+#pragma unroll
+    for (int w = 0; w < kSampleThreads / 32; ++w) {
+      const int x = s_scan[w];
+      if (w < warp) upto += x;
+      total += x;
+    }
+    if (upto >= want && upto - mine < want) {
+      int above = upto - mine, bin = 0;
+      bool found = false;
+#pragma unroll
+      for (int i = PER - 1; i >= 0; --i) {
+        if (found) continue;
+        if (i == 0 || above + q[0][i] >= want) {
+          bin = i;
+          found = true;
+        } else {
+          above += q[0][i];
+        }
+      }
+      s_bin = static_cast<uint32_t>(first + bin);
+      s_above = above;
     }
     __syncthreads();
+    return total >= want;
+  };
+  uint32_t thr = 0;  // fewer groups than C with anything in them: every allowed logit
+  if (find_bin(std::integral_constant<int, kBins / kSampleThreads>(), s_hist, C)) {
+    const uint32_t top = s_bin;
+    const int above = s_above;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (gm[e] != 0 && gm[e] >> 21 == top) atomicAdd(&s_hist2[(gm[e] >> 11) & (kBins2 - 1)], 1);
+    find_bin(std::integral_constant<int, kBins2 / kSampleThreads>(), s_hist2, C - above);
+    thr = (top << 21) | (s_bin << 11);
+  } else {
+    cluster.sync();  // the same barriers on either way
   }
 
-  // ---- filters and draw (serial over <= 1024 sorted candidates) ----
-  if (threadIdx.x == 0) {
-    if (n <= 0) {
-      p.out_tokens[row] = 0;
-      return;
-    }
-    const float inv_t = 1.f / temp;
-    const float mx = s_val[0] * inv_t;
-    float sum = 0.f;
-    for (int i = 0; i < n; ++i) {
-      const float e = __expf(s_val[i] * inv_t - mx);
-      s_val[i] = e;
-      sum += e;
-    }
-    if (full_mass) sum = fmaxf(sum, s_best);
-    // min-p: keep probabilities >= min_p * p_max (p_max is candidate 0)
-    int keep = n;
-    if (min_p > 0.f) {
-      const float thr = min_p * s_val[0];
-      int c = 0;
-      while (c < n && s_val[c] >= thr) ++c;
-      keep = c > 0 ? c : 1;
-    }
-    if (top_k < keep) keep = top_k;
-    // top-p: cumulative mass of the candidate softmax (not renormalised after min-p / top-k,
-    // as in the reference pipeline)
-    if (top_p < 1.f) {
-      float cum = 0.f;
-      int c = 0;
-      while (c < keep) {
-        cum += s_val[c] / sum;
-        ++c;
-        if (cum >= top_p) break;
-      }
-      keep = c > 0 ? c : 1;
-    }
-    float tot = 0.f;
-    for (int i = 0; i < keep; ++i) tot += s_val[i];
-    const uint64_t seed = p.seeds != nullptr ? p.seeds[row] : 0ull;
-    const uint64_t ctr = p.counters != nullptr ? p.counters[row] : 0ull;
-    const uint64_t r = splitmix64(seed ^ splitmix64(ctr + 0x51ED2701ull));
-    const float u = static_cast<float>(r >> 40) * (1.0f / 16777216.0f);
-    const float target = u * tot;
-    float cum = 0.f;
-    int pick = keep - 1;
-    for (int i = 0; i < keep; ++i) {
-      cum += s_val[i];
-      if (cum > target) {
-        pick = i;
-        break;
+  // ---- 2. gather ----
+  const float thr_f = thr == 0 ? -INFINITY : key2f(thr);
+  auto give = [&](float x, int i) {
+    if (x < thr_f) return;
+    const int at = atomicAdd(&s_count, 1);
+    if (at < kSampleCap) s_cand[at] = cand_word(x, i);
+  };
+  if (thr == 0 || gm[0] >= thr || gm[1] >= thr || gm[2] >= thr || gm[3] >= thr) {
+    for (int v = v_lo + tid; v < v_fast; v += kBatch * kSampleThreads) {
+      float4 x[kBatch];
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u)
+        x[u] = v + u * kSampleThreads < v_fast ? __ldcg(reinterpret_cast<const float4*>(logits) + v + u * kSampleThreads) : none;
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        const int i = 4 * (v + u * kSampleThreads);
+        if (i >= 4 * v_fast) continue;
+        give(x[u].x, i);
+        give(x[u].y, i + 1);
+        give(x[u].z, i + 2);
+        give(x[u].w, i + 3);
       }
     }
-    p.out_tokens[row] = s_idx[pick];
-    if (p.out_logit != nullptr) p.out_logit[row] = logf(s_val[pick] / sum);
+    for (int v = v_fast + tid; v < v_hi; v += kSampleThreads) {
+      float y[4];
+      uint32_t ok;
+      load4(v, y, ok);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if ((ok >> e) & 1u) give(y[e], 4 * v + e);
+    }
+  }
+  if (full_mass) {
+    // the threads' sums relative to the largest logit of their warp
+    float m = run_m;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float part = warp_sum(m == -INFINITY ? 0.f : run_s * __expf(run_m * inv_t - m * inv_t));
+    if (lane == 0) {
+      s_fscan[warp] = part;
+      s_fmax[warp] = m;
+    }
+  }
+  __syncthreads();
+  // every CTA sends its candidates to the first one
+  const int found = s_count;
+  if (tid == 0) {
+    s_base = atomicAdd(cluster.map_shared_rank(&s_total, 0), found);
+  }
+  if (full_mass && warp == 1) {
+    const float x = lane < kSampleThreads / 32 ? s_fmax[lane] : -INFINITY;
+    float m = x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float t = warp_sum(lane < kSampleThreads / 32 && x != -INFINITY ? s_fscan[lane] * __expf(x * inv_t - m * inv_t) : 0.f);
+    if (lane == 0) {
+      cluster.map_shared_rank(s_part, 0)[rank] = t;
+      cluster.map_shared_rank(s_part_max, 0)[rank] = m;
+    }
+  }
+  __syncthreads();
+  {
+    unsigned long long* to = cluster.map_shared_rank(s_sort, 0);
+    const int base = s_base;
+    for (int i = tid; i < found && i < kSampleCap && base + i < kSampleCap; i += kSampleThreads) to[base + i] = s_cand[i];
+  }
+  cluster.sync();
+  if (rank != 0) return;
+  int n = s_total;
+
+  // ---- 3. sort, filter, draw ----
+  if (n > kSampleCap) n = select_exact(logits, mask, V, C, s_hist, s_sort);
+  if (n <= 0) {
+    if (tid == 0) p.out_tokens[row] = 0;
+    return;
+  }
+  if (n <= kSampleThreads) {
+    // every thread counts the words that come before its own
+    const unsigned long long mine = tid < n ? s_sort[tid] : 0;
+    if (tid == 0) s_sort[n] = 0;
+    __syncthreads();
+    int before = 0;
+    for (int i = 0; i < n; i += 2) {
+      const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(s_sort + i);
+      before += (w.x > mine) + (w.y > mine);
+    }
+    __syncthreads();
+    if (tid < n) s_sort[before] = mine;
+  } else {
+    // bitonic, descending; with a distance of up to 32 the 32 pairs of a warp lie in 64 words of its own
+    int P = kSampleThreads;
+    while (P < n) P <<= 1;
+    for (int i = n + tid; i < P; i += kSampleThreads) s_sort[i] = 0;
+    __syncthreads();
+    for (int k = 2; k <= P; k <<= 1) {
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int q = tid; q < P / 2; q += kSampleThreads) {
+          const int i = 2 * q - (q & (j - 1));
+          const unsigned long long a = s_sort[i], b = s_sort[i + j];
+          if ((i & k) == 0 ? a < b : a > b) {
+            s_sort[i] = b;
+            s_sort[i + j] = a;
+          }
+        }
+        if (j > 32 || (j == 1 && k >= 64)) __syncthreads();
+        else __syncwarp();
+      }
+    }
+  }
+  __syncthreads();
+  if (n > C) n = C;
+
+  // softmax numerators of candidates 2 tid and 2 tid + 1, and their running sums
+  float ev[2], cum[2];
+  const float m0 = key2f(static_cast<uint32_t>(s_sort[0] >> 32)) * inv_t;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int i = 2 * tid + e;
+    ev[e] = i < n ? __expf(key2f(static_cast<uint32_t>(s_sort[i] >> 32)) * inv_t - m0) : 0.f;
+  }
+  float run = ev[0] + ev[1];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float q = __shfl_up_sync(0xffffffffu, run, o);
+    if (lane >= o) run += q;
+  }
+  if (lane == 31) s_fscan[warp] = run;
+  float before = __shfl_up_sync(0xffffffffu, run, 1);
+  if (lane == 0) before = 0.f;
+  if (tid == 0) {
+    s_best = ev[0];
+    s_first = n;
+  }
+  __syncthreads();
+  float sum = 0.f;
+#pragma unroll
+  for (int w = 0; w < kSampleThreads / 32; ++w) {
+    if (w == warp) before += sum;
+    sum += s_fscan[w];
+  }
+  cum[0] = before + ev[0];
+  cum[1] = cum[0] + ev[1];
+  if (full_mass) {
+    float mass = 0.f;
+    for (int r = 0; r < S; ++r) mass += s_part_max[r] == -INFINITY ? 0.f : s_part[r] * __expf(s_part_max[r] * inv_t - m0);
+    sum = fmaxf(sum, mass);
+  }
+  // the first candidate below `n` for which `hit` holds, else n
+  auto first_of = [&](int limit, auto hit) -> int {
+    if (tid == 0) s_first = limit;
+    __syncthreads();
+    int mine = limit;
+#pragma unroll
+    for (int e = 1; e >= 0; --e)
+      if (2 * tid + e < limit && hit(e)) mine = 2 * tid + e;
+    mine = __reduce_min_sync(0xffffffffu, mine);
+    if (lane == 0 && mine < limit) atomicMin(&s_first, mine);
+    __syncthreads();
+    const int r = s_first;
+    __syncthreads();
+    return r;
+  };
+  int keep = n;
+  // min-p: keep probabilities >= min_p * p_max (p_max is candidate 0)
+  if (min_p > 0.f) {
+    const float least = min_p * s_best;
+    keep = first_of(n, [&](int e) { return !(ev[e] >= least); });
+    if (keep < 1) keep = 1;
+  }
+  if (top_k < keep) keep = top_k;
+  // top-p: cumulative mass of the candidate softmax (not renormalised after min-p / top-k,
+  // as in the reference pipeline)
+  if (top_p < 1.f) {
+    const int c = first_of(keep, [&](int e) { return cum[e] / sum >= top_p; });
+    if (c < keep) keep = c + 1;
+  }
+  if ((keep - 1) >> 1 == tid) s_tot = cum[(keep - 1) & 1];
+  __syncthreads();
+  const uint64_t seed = p.seeds != nullptr ? p.seeds[row] : 0ull;
+  const uint64_t ctr = p.counters != nullptr ? p.counters[row] : 0ull;
+  const uint64_t r = splitmix64(seed ^ splitmix64(ctr + 0x51ED2701ull));
+  const float u = static_cast<float>(r >> 40) * (1.0f / 16777216.0f);
+  const float target = u * s_tot;
+  int pick = first_of(keep, [&](int e) { return cum[e] > target; });
+  if (pick >= keep) pick = keep - 1;
+  if (pick >> 1 == tid) {
+    p.out_tokens[row] = static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(s_sort[pick]));
+    if (p.out_logit != nullptr) p.out_logit[row] = logf(ev[pick & 1] / sum);
   }
 }
 
@@ -286,7 +585,7 @@ __global__ void __launch_bounds__(kThreads) argmax_kernel(const float* logits, l
                                                           int* out, float* out_val) {
   __shared__ int s_tok;
   __shared__ float s_best;
-  block_argmax(logits + static_cast<long long>(blockIdx.x) * ld, nullptr, V, &s_tok, &s_best);
+  block_argmax(logits + static_cast<long long>(blockIdx.x) * ld, V, &s_tok, &s_best);
   if (threadIdx.x == 0) {
     out[blockIdx.x] = s_tok;
     if (out_val != nullptr) out_val[blockIdx.x] = s_best;
@@ -315,7 +614,7 @@ __global__ void __launch_bounds__(kThreads) argmax_push_kernel(const ArgmaxExcha
   __shared__ int s_tok;
   __shared__ float s_best;
   const int row = blockIdx.x;
-  block_argmax(p.logits + static_cast<long long>(row) * p.ld, nullptr, p.V_local, &s_tok, &s_best);
+  block_argmax(p.logits + static_cast<long long>(row) * p.ld, p.V_local, &s_tok, &s_best);
   if (threadIdx.x == 0) {
     const unsigned long long word = (static_cast<unsigned long long>(f2key(s_best)) << 32) |
                                     (0xFFFFFFFFu - static_cast<uint32_t>(s_tok + p.vocab_start));
@@ -361,7 +660,22 @@ void launch_argmax_exchange(const ArgmaxExchangeParams& p, cudaStream_t stream) 
 
 void launch_sample(const SampleParams& p, int rows, cudaStream_t stream) {
   if (rows <= 0) return;
-  sample_kernel<<<rows, kThreads, 0, stream>>>(p);
+  // as many CTAs per row as are resident at once (two per SM; clusters of a second wave would start when the first is done), of at
+  // least 4096 logits each (two loads per thread; fewer do not pay for a barrier across the cluster)
+  int S = kMaxSlices;
+  while (S > 1 && (static_cast<long long>(rows) * S > 2ll * sm_count() || p.V < S * 4096)) S >>= 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows) * S);
+  cfg.blockDim = dim3(kSampleThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = S;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, sample_kernel, p);
 }
 void launch_argmax(const float* logits, long long ld, int V, int rows, int* out, float* out_val,
                    cudaStream_t stream) {

@@ -926,6 +926,78 @@ def test_argmax_and_sampling(ops):
     torch.testing.assert_close(lp, torch.log(full[toks.long()]), rtol=0, atol=2e-3)
 
 
+def _splitmix64(x):
+    x = (x + 0x9E3779B97F4A7C15) & (2 ** 64 - 1)
+    x = ((x ^ (x >> 30)) * 0xBF58476D1CE4E5B9) & (2 ** 64 - 1)
+    x = ((x ^ (x >> 27)) * 0x94D049BB133111EB) & (2 ** 64 - 1)
+    return x ^ (x >> 31)
+
+
+@pytest.mark.parametrize("rows,vocab,pad,top_k,top_p,min_p,kind", [
+    (1, 128256, 0, 50, 0.95, 0.0, "bell"), (3, 32003, 1, 0, 0.9, 0.0, "bell"), (70, 9001, 3, 700, 1.0, 0.02, "bell"),
+    (200, 32000, 0, 0, 0.8, 0.05, "bell"), (2, 300, 0, 5, 1.0, 0.0, "bell"), (2, 7, 1, 3, 0.9, 0.0, "bell"), (400, 4099, 1, 20, 0.9, 0.0, "bell"),
+    (2, 50000, 0, 50, 0.95, 0.0, "equal"), (2, 50000, 0, 0, 0.5, 0.0, "steps"), (5, 40000, 0, 0, 0.9, 0.0, "mask"), (5, 40000, 2, 100, 1.0, 0.0, "few"),
+    (2, 30000, 0, 100, 1.0, 0.0, "sorted"), (3, 8192, 0, 40, 1.0, 0.0, "lowest")])
+def test_sample_against_sorted_rows(ops, rows, vocab, pad, top_k, top_p, min_p, kind):
+    """The draw of every row against the filters on the sorted row in 64 bits: all slice counts, unaligned rows, ties, masks."""
+    g = torch.Generator().manual_seed(vocab + rows)
+    x = torch.randn(rows, vocab, generator=g) * 2.5
+    allow = torch.ones(rows, vocab, dtype=torch.bool)
+    if kind == "equal":
+        x[:] = 1.25                                   # thousands of equal logits: the exact selection
+    elif kind == "steps":
+        x = (x * 2).round() / 2
+    elif kind == "sorted":
+        x = x.sort(-1, descending=True).values
+    elif kind == "lowest":
+        x[:, 10:] = -math.inf                         # fewer finite logits than candidates
+    elif kind in ("mask", "few"):
+        allow = torch.rand(rows, vocab, generator=g) < (0.3 if kind == "mask" else 0.001)
+        allow[:, 17] = True
+    temp, seed = 0.7, torch.randint(0, 1 << 62, (rows,), generator=g)
+    wide = torch.full((rows, vocab + pad), math.inf, device=DEV)
+    wide[:, :vocab] = x.to(DEV)
+    bits = torch.zeros(rows, (vocab + 31) // 32 * 32, dtype=torch.int64)
+    bits[:, :vocab] = allow
+    words = (bits.view(rows, -1, 32) << torch.arange(32)).sum(-1)
+    mask = torch.where(words >= 1 << 31, words - (1 << 32), words).to(torch.int32).to(DEV)
+    full = lambda v, dt: torch.full((rows,), v, dtype=dt, device=DEV)
+    out, lp = full(-1, torch.int32), full(0.0, torch.float32)
+    args = dict(temperature=full(temp, torch.float32), top_k=full(top_k, torch.int32), top_p=full(top_p, torch.float32),
+                min_p=full(min_p, torch.float32), seeds=seed.to(DEV), counters=torch.arange(rows, device=DEV),
+                allow_mask=mask if kind in ("mask", "few") else None)
+    ops.sample(wide[:, :vocab], out, out_logit=lp, **args)
+    greedy = full(-1, torch.int32)
+    ops.sample(wide[:, :vocab], greedy, **{**args, "temperature": full(0.0, torch.float32)})
+    torch.cuda.synchronize()
+    ranked = torch.where(allow, x, -math.inf)
+    assert torch.equal(greedy.cpu().long(), ranked.max(-1).indices) or kind in ("equal", "steps")
+    for b in range(rows):
+        assert float(ranked[b, greedy[b]]) == float(ranked[b].max())
+        at = allow[b].nonzero().flatten()
+        v, order = x[b, at].double().sort(descending=True, stable=True)
+        k = top_k if 0 < top_k < vocab else vocab
+        n = min(max(k, 256), 1024, len(at))
+        e = torch.exp((v - v[0]) / temp)
+        total = float(e.sum()) if k == vocab and vocab > min(max(k, 256), 1024) else float(e[:n].sum())
+        e = e[:n]
+        keep = min(k, int((e >= min_p).sum()) if min_p > 0 else n)
+        cum = e.cumsum(0)
+        edges = [cum / total - top_p] if top_p < 1 else []
+        if top_p < 1:
+            keep = min(keep, int((cum / total < top_p).sum()) + 1)
+        u = (_splitmix64(int(seed[b]) ^ _splitmix64(b + 0x51ED2701)) >> 40) / 2 ** 24
+        edges.append((cum - u * cum[keep - 1]) / cum[keep - 1])
+        pick = min(int((cum[:keep] <= u * cum[keep - 1]).sum()), keep - 1)
+        # 32-bit sums of up to 1024 terms are off by less than 1024 * 2^-24: closer draws may fall on the neighbour
+        if min(float(d.abs().min()) for d in edges) < 6e-5:
+            continue
+        if kind not in ("equal", "steps", "lowest"):   # which of several equal logits at the C-th place is open
+            assert int(out[b]) == int(at[order[pick]]), (b, pick)
+        assert float(x[b, out[b]]) == float(v[pick])
+        assert abs(float(lp[b]) - math.log(float(e[pick]) / total)) < 2e-4
+
+
 def test_argmax_exchange_on_one_rank(ops):
     """The peer-memory argmax exchange with a single rank: the word table is this GPU's own, both slots
     give the argmax (lowest index on ties) and leave the table empty; a word that never arrives ends
