@@ -1,0 +1,438 @@
+// tcgen05 GEMM of a few activation rows with GGUF-packed weights (Q4_K, Q5_K, Q6_K):  out[m, n] += sum_k x[m, k] W[n, k], M <= 256.
+//
+// The weights are the rows of the MMA (M = 128 weight rows, N = activation rows padded to 16), so a small batch costs what its rows
+// cost, and they go from registers to TMEM, where the MMA takes them from: a lane of TMEM is a weight row, a thread unpacks the 256
+// values of one super-block of its own row, and nothing is swizzled or written to shared memory on the way. The packed blocks
+// themselves arrive by TMA (a box of 128 rows x one super-block), ahead of everything else.
+//
+// Persistent. The units of work are (128 weight rows) x (256 values of K); every CTA takes an equal, contiguous run of them, which may
+// begin and end inside a row of units: all results are added to `out` in fp32, so K is split wherever a run ends and there
+// is no last wave. Warps: 0 = packed weights (TMA), 18 = activations (TMA), 1 = TMEM owner and MMA issuer, 6..17 = three groups of
+// four that unpack every third unit, 2..5 = epilogue. Every wait is bounded.
+//
+// What bounds it: the instructions that unpack (about 3.5 per weight, two operations in most; 65536 x 8192 of Q6_K and 57344 x 8192 of
+// Q4_K with 32 rows: 127 and 98 us, 3.5 and 2.7 TB/s of packed bytes; with 128 rows 160 and 133). Weights unpacked into shared memory as
+// the columns of a 128-row MMA by four warps that load their own blocks (the other types, gemm_bf16.cu) take 700 us there: each
+// unpacked byte crosses shared memory twice, and the loads of a block wait for the last one's stores.
+#include "gemm_unpack.cuh"
+
+#include <type_traits>
+
+#include "../common/device_info.h"
+#include "../common/sm100.cuh"
+#include "quant_blocks.cuh"
+
+namespace oxb {
+
+namespace {
+
+constexpr int kTileN = 128;       // weight rows of a tile: lanes of TMEM
+constexpr int kSuper = 256;       // values of K per unit: one super-block
+constexpr int kGroups = 3;        // of four warps that unpack, one per unpacked unit in TMEM
+constexpr int kUnpackThreads = 32 * (7 + 4 * kGroups);
+constexpr int kXWarp = 6 + 4 * kGroups;
+constexpr int kMaxRing = 24;
+
+template <int T>
+struct Super;  // bytes of a super-block; bytes of a TMA box row that holds one from a 16-byte boundary on (an odd multiple of 16
+               // keeps 16-byte reads of 8 neighbouring rows free of bank conflicts)
+template <>
+struct Super<kQ_Q4_K> {
+  static constexpr int kBytes = 144, kBox = 144;
+};
+template <>
+struct Super<kQ_Q5_K> {
+  static constexpr int kBytes = 176, kBox = 176;
+};
+template <>
+struct Super<kQ_Q6_K> {
+  static constexpr int kBytes = 210, kBox = 240;  // 2-byte aligned: up to 14 bytes before it
+};
+
+__device__ __forceinline__ float byte_float(uint32_t w, int i) {  // byte i of w as a float, exactly
+  return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650 + i)) - 8388608.f;
+}
+// Four codes q_i, placed under the implicit one of a float's mantissa (byte i of `t` is bits 16..23 of 2^e + q_i, `top` its bits
+// 24..31), times dl plus c, as two words of bf16 pairs. c takes back dl * 2^e.
+__device__ __forceinline__ void four(uint32_t t, uint32_t top, float dl, float c, uint32_t& w0, uint32_t& w1) {
+  const float2 d2 = make_float2(dl, dl), c2 = make_float2(c, c);
+  const float2 a = fma_f32x2(make_float2(__uint_as_float(__byte_perm(t, top, 0x7054)), __uint_as_float(__byte_perm(t, top, 0x7154))), d2, c2);
+  const float2 b = fma_f32x2(make_float2(__uint_as_float(__byte_perm(t, top, 0x7254)), __uint_as_float(__byte_perm(t, top, 0x7354))), d2, c2);
+  w0 = pack_bf16x2(a.x, a.y);
+  w1 = pack_bf16x2(b.x, b.y);
+}
+// N words from the 2-byte aligned place `off` (0, 2, 4 or 6) bytes behind the 8-byte aligned `p`. `off` is the same in all lanes.
+template <int N>
+__device__ __forceinline__ void words_at(const uint8_t* p, int off, uint32_t (&w)[N]) {
+  constexpr int kPairs = (N + 3) / 2;
+  uint32_t r[2 * kPairs];
+#pragma unroll
+  for (int i = 0; i < kPairs; ++i) {
+    const uint2 x = reinterpret_cast<const uint2*>(p)[i];
+    r[2 * i] = x.x;
+    r[2 * i + 1] = x.y;
+  }
+  const uint32_t sel = (off & 2) ? 0x5432u : 0x3210u;
+  if (off & 4) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __byte_perm(r[i + 1], r[i + 2], sel);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __byte_perm(r[i], r[i + 1], sel);
+  }
+}
+
+// The super-block whose box row starts at `b` (and itself `off` bytes later) -> 8 x 16 words of bf16 pairs; `put(i, w)` takes values
+// [32 i, 32 i + 32).
+template <int T, typename Put>
+__device__ __forceinline__ void unpack_super(const uint8_t* b, int off, Put put) {
+  if constexpr (T == kQ_Q4_K || T == kQ_Q5_K) {
+    // d | dmin | 12 bytes of 6-bit scales and minima | (Q5_K: 32 bytes of fifth bits) | 128 bytes of nibbles
+    const uint4 hdr = *reinterpret_cast<const uint4*>(b);
+    const __half2 dm = *reinterpret_cast<const __half2*>(&hdr.x);
+    const float d = __low2float(dm), dmin = __high2float(dm);
+    const uint32_t sc[2] = {hdr.y & 0x3F3F3F3Fu, (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u)};
+    const uint32_t mn[2] = {hdr.z & 0x3F3F3F3Fu, ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u)};
+    uint4 ha = make_uint4(0, 0, 0, 0), hb = ha;
+    if constexpr (T == kQ_Q5_K) {
+      ha = reinterpret_cast<const uint4*>(b + 16)[0];
+      hb = reinterpret_cast<const uint4*>(b + 16)[1];
+    }
+    const uint32_t h[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint4* q = reinterpret_cast<const uint4*>(b + (T == kQ_Q4_K ? 16 : 48) + j * 32);
+      const uint4 qa = q[0], qb = q[1];
+      const uint32_t n[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {  // 32 values: low, then high nibbles
+        uint32_t w[16];
+        const int sub = 2 * j + g;
+        const float dl = d * byte_float(sc[sub >> 2], sub & 3);
+        const float ml = -dmin * byte_float(mn[sub >> 2], sub & 3);
+        if constexpr (T == kQ_Q4_K) {
+          const float c = fmaf(-16.f, dl, ml);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            four(((g == 0 ? n[u] << 3 : n[u] >> 1) & 0x78787878u) | 0x80808080u, 0x41000000u, dl, c, w[2 * u], w[2 * u + 1]);
+        } else {
+          const float c = fmaf(-32.f, dl, ml);
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            four(((g == 0 ? n[u] << 2 : n[u] >> 2) & 0x3C3C3C3Cu) | ((sub <= 6 ? h[u] << (6 - sub) : h[u] >> 1) & 0x40404040u), 0x42000000u, dl, c,
+                 w[2 * u], w[2 * u + 1]);
+        }
+        put(sub, w);
+      }
+    }
+  } else {
+    // 128 bytes of nibbles | 64 of upper bit pairs | 16 signed scales | d
+    const uint8_t* p = b + (off & 8);
+    off &= 7;
+    uint32_t sw[5];
+    words_at<5>(p + 192, off, sw);
+    const float d = __half2float(__ushort_as_half(static_cast<uint16_t>(sw[4] & 0xFFFFu)));
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint32_t lo[16], hi[8];
+      words_at<16>(p + 64 * half, off, lo);
+      words_at<8>(p + 128 + 32 * half, off, hi);
+#pragma unroll
+      for (int pi = 0; pi < 2; ++pi) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          uint32_t w[16];
+          const int hs = 4 * pi + 2 * g;  // place of the upper bits, to go to bits 5 and 6
+          const uint32_t s4 = sw[2 * half + pi] ^ 0x80808080u;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {  // 16 values per scale
+            const float dl = d * (byte_float(s4, 2 * g + k) - 128.f);
+            const float c = -96.f * dl;  // exact: 64 of the float's own, 32 of the code's offset
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const int u = 4 * k + v;
+              const uint32_t l = lo[8 * g + u], x = hi[u];
+              const uint32_t t = ((pi == 0 ? l << 1 : l >> 3) & 0x1E1E1E1Eu) | ((hs <= 5 ? x << (5 - hs) : x >> (hs - 5)) & 0x60606060u) | 0x80808080u;
+              four(t, 0x42000000u, dl, c, w[2 * u], w[2 * u + 1]);
+            }
+          }
+          put(4 * half + 2 * pi + g, w);
+        }
+      }
+    }
+  }
+}
+
+template <int T>
+__global__ void __launch_bounds__(kUnpackThreads, 1)
+gemm_unpack_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const GemmUnpackParams p) {
+  constexpr int kStageW = kTileN * Super<T>::kBox;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int box_x = p.m_pad * 128;  // activation rows x 64 values
+  const int stage_x = p.x_boxes * box_x;
+  uint8_t* sX = smem;
+  uint8_t* sW = smem + p.x_stages * stage_x;
+  uint64_t* w_full = reinterpret_cast<uint64_t*>(sW + p.w_stages * kStageW);
+  uint64_t* w_empty = w_full + kMaxRing;
+  uint64_t* x_full = w_empty + kMaxRing;
+  uint64_t* x_empty = x_full + kMaxRing;
+  uint64_t* a_full = x_empty + kMaxRing;   // [3] unpacked units in TMEM
+  uint64_t* a_empty = a_full + 3;
+  uint64_t* d_full = a_empty + 3;          // [2]
+  uint64_t* d_empty = d_full + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(d_empty + 2);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t spin = spin_budget(p.spin_limit);
+  const int n_kb = p.K / kSuper;
+  const long long units = static_cast<long long>((p.N + kTileN - 1) / kTileN) * n_kb;
+  const long long u_lo = units * blockIdx.x / gridDim.x, u_hi = units * (blockIdx.x + 1) / gridDim.x;
+  const int n_units = static_cast<int>(u_hi - u_lo);
+  const int tile0 = static_cast<int>(u_lo / n_kb), kb_first = static_cast<int>(u_lo - static_cast<long long>(tile0) * n_kb);
+  // Place of a role in the run of units: nothing is divided on the way, a division costs as much as unpacking 30 values.
+  struct Place {
+    int tile, kb, n_kb;
+    __device__ __forceinline__ void next() {
+      if (++kb == n_kb) {
+        kb = 0;
+        ++tile;
+      }
+    }
+  };
+  struct Ring {  // slot of a ring and the parity of its current use
+    int slot = 0;
+    uint32_t parity = 0;
+    bool first = true;
+    __device__ __forceinline__ void next(int size) {
+      if (++slot == size) {
+        slot = 0;
+        parity ^= 1;
+        first = false;
+      }
+    }
+  };
+  Place at{tile0, kb_first, n_kb};
+  // TMEM: accumulators from column 0 (two of them up to 64 rows), then the unpacked units of 128 columns
+  const int n_acc = p.m_pad <= 64 ? 2 : 1;
+  const int n_a = p.m_pad <= 128 ? kGroups : 2;
+  const uint32_t a_col = p.m_pad <= 128 ? 128 : 256;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+    for (int i = 0; i < p.w_stages; ++i) {
+      mbar_init(&w_full[i], 1);
+      mbar_init(&w_empty[i], 4);
+    }
+    for (int i = 0; i < p.x_stages; ++i) {
+      mbar_init(&x_full[i], 1);
+      mbar_init(&x_empty[i], 1);
+    }
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(&a_full[i], 4);
+      mbar_init(&a_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&d_full[i], 1);
+      mbar_init(&d_empty[i], 4);
+    }
+    fence_mbar_init();
+  }
+  __syncthreads();
+  // TMEM is taken only when the prerequisite grid is done (it may be in use on this SM until then); the weights
+  // depend on nothing that runs before this kernel
+  uint32_t tmem_base = 0;
+  if (warp >= 1 && warp < kXWarp) {
+    pdl_wait();
+    if (warp == 1) {
+      tmem_alloc(tmem_slot, 512);
+      tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    asm volatile("bar.sync 2, %0;" ::"n"(32 * (kXWarp - 1)) : "memory");
+    tc_fence_after_sync();
+    tmem_base = *tmem_slot;
+  }
+
+  if (warp == 0) {
+    // ------------------------------ packed weights ----------------------------
+    // one lane per stage: copies that one thread issues complete one after the other
+    Ring r;
+    bool ok = true;
+    for (int it = 0; it < n_units; ++it, at.next(), r.next(p.w_stages)) {
+      if (!r.first && !mbar_wait(&w_empty[r.slot], r.parity ^ 1, spin)) ok = false;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutProducer);
+        break;
+      }
+      if (lane == r.slot) {
+        mbar_arrive_expect_tx(&w_full[r.slot], kStageW);
+        tma_load_2d(sW + r.slot * kStageW, &tmW, &w_full[r.slot], (at.kb * Super<T>::kBytes & ~15) / 2, at.tile * kTileN);
+      }
+      __syncwarp();
+    }
+  } else if (warp == kXWarp) {
+    // ------------------------------ activations -------------------------------
+    pdl_wait();
+    Ring r;
+    bool ok = true;
+    for (int it = 0; it < n_units && ok; ++it, at.next()) {
+      for (int c = 0; c < 4; c += p.x_boxes, r.next(p.x_stages)) {
+        if (!r.first && !mbar_wait(&x_empty[r.slot], r.parity ^ 1, spin)) ok = false;
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutProducer);
+          break;
+        }
+        if (lane == 0) mbar_arrive_expect_tx(&x_full[r.slot], stage_x);
+        __syncwarp();
+        const int b = lane - 4 * (r.slot & 7);  // a lane per box, other lanes for the next stage
+        if (b >= 0 && b < p.x_boxes)
+          tma_load_2d(sX + r.slot * stage_x + b * box_x, &tmX, &x_full[r.slot], at.kb * kSuper + (c + b) * 64, 0);
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer --------------------------------
+    // The whole warp walks and waits, an elected lane issues. With the loop inside a branch on the lane index each MMA took 125
+    // clocks to issue, three times its work at 32 rows.
+    const uint32_t idesc = make_idesc(kFmtBF16, kFmtBF16, kTileN, static_cast<uint32_t>(p.m_pad));
+    const uint64_t x_desc = make_desc_kmajor_sw128(smem_u32(sX));  // addresses in a descriptor count 16 bytes
+    Ring rx, ra, rd;
+    bool ok = true;
+    for (int it = 0; it < n_units && ok; rd.next(n_acc)) {
+      if (!rd.first && !mbar_wait(&d_empty[rd.slot], rd.parity ^ 1, spin)) ok = false;
+      const int end = it + (n_kb - at.kb) < n_units ? it + (n_kb - at.kb) : n_units;
+      const uint32_t d = tmem_base + rd.slot * 64;
+      uint32_t more = 0;
+      for (; it < end && ok; ++it, at.next(), ra.next(n_a)) {
+        if (!mbar_wait(&a_full[ra.slot], ra.parity, spin)) ok = false;
+        for (int c = 0; c < 4; c += p.x_boxes, rx.next(p.x_stages)) {
+          if (ok && !mbar_wait(&x_full[rx.slot], rx.parity, spin)) ok = false;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after_sync();
+          const uint64_t x = x_desc + static_cast<uint32_t>(rx.slot * stage_x) / 16;
+          const uint32_t a = tmem_base + a_col + ra.slot * 128 + c * 32;
+          if (elect_one()) {
+            for (int b = 0; b < p.x_boxes; ++b) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                tc_mma_f16_ts(d, a + b * 32 + k * 8, x + static_cast<uint32_t>(b * box_x + k * 32) / 16, idesc, more | static_cast<uint32_t>(b + k));
+            }
+            tc_commit(&x_empty[rx.slot]);
+            if (c + p.x_boxes >= 4) tc_commit(&a_empty[ra.slot]);
+          }
+          __syncwarp();
+          more = 1;
+        }
+      }
+      if (ok && elect_one()) tc_commit(&d_full[rd.slot]);
+      __syncwarp();
+    }
+    if (!ok && lane == 0) set_status_once(p.status, kStatusMbarTimeoutMma);
+    if (lane == 0) pdl_launch_dependents();
+  } else if (warp >= 6) {
+    // ------------------------------ unpacking ---------------------------------
+    const int q = warp & 3;  // TMEM lane quarter of this warp
+    const int row = q * 32 + lane;
+    const int group = (warp - 6) >> 2;
+    Ring rw, ra;
+    bool ok = true;
+    for (int it = 0; it < n_units; ++it, at.next(), rw.next(p.w_stages), ra.next(n_a)) {
+      if (ra.slot != group) continue;  // (the third group has no units when only two fit)
+      // In this order: a parity tells neighbouring uses of a barrier apart, no more. The place in TMEM is this group's own, and when it is
+      // empty the n_a-th unit before this one has been multiplied, so all earlier ones have arrived and none of the weight
+      // ring's barriers (w_stages >= n_a) is two uses behind.
+      if (!ra.first && !mbar_wait(&a_empty[ra.slot], ra.parity ^ 1, spin)) ok = false;
+      if (ok && !mbar_wait(&w_full[rw.slot], rw.parity, spin)) ok = false;
+      ok = __all_sync(0xffffffffu, ok);  // tcgen05.st below is warp-collective
+      if (!ok) {
+        if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutProducer);
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t to = tmem_base + a_col + ra.slot * 128 + (static_cast<uint32_t>(q * 32) << 16);
+      unpack_super<T>(sW + rw.slot * kStageW + row * Super<T>::kBox, at.kb * Super<T>::kBytes & 15,
+                      [&](int i, const uint32_t (&w)[16]) __attribute__((always_inline)) { tmem_st_32x32b_x16(to + i * 16, w); });
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&a_full[ra.slot]);
+        mbar_arrive(&w_empty[rw.slot]);
+      }
+    }
+  } else {
+    // ------------------------------ epilogue ----------------------------------
+    const int q = warp & 3;
+    Ring rd;
+    bool ok = true;
+    for (int it = 0; it < n_units; rd.next(n_acc)) {
+      ok = mbar_wait(&d_full[rd.slot], rd.parity, spin);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutEpilogue);
+        break;
+      }
+      tc_fence_after_sync();
+      const int n = at.tile * kTileN + q * 32 + lane;  // lane = output column
+      it += n_kb - at.kb;
+      at.kb = 0;
+      ++at.tile;
+      for (int c = 0; c < p.M; c += 32) {
+        uint32_t v[32];
+        tmem_ld_32x32b_x32(tmem_base + rd.slot * 64 + c + (static_cast<uint32_t>(q * 32) << 16), v);
+        tmem_ld_wait();
+        if (n >= p.N) continue;
+        float* d = p.out + static_cast<long long>(c) * p.ldo + n;
+#pragma unroll
+        for (int j = 0; j < 32; ++j, d += p.ldo)
+          if (c + j < p.M) atomicAdd(d, __uint_as_float(v[j]));
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&d_empty[rd.slot]);
+    }
+    tc_fence_before_sync();
+  }
+
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+template <int T>
+void launch_type(const CUtensorMap& tmW, const CUtensorMap& tmX, GemmUnpackParams p, cudaStream_t stream) {
+  constexpr int kBars = (4 * kMaxRing + 10) * 8 + 16, kBudget = 226 * 1024;
+  constexpr int kStageW = kTileN * Super<T>::kBox;
+  // activations in stages of a super-block where they are small (each stage costs the issuing thread a wait and a commit), the
+  // packed weights take the rest
+  p.x_boxes = p.m_pad <= 64 ? 4 : (p.m_pad <= 128 ? 2 : 1);
+  p.x_stages = 3;
+  p.w_stages = (kBudget - 1024 - kBars - p.x_stages * p.x_boxes * p.m_pad * 128) / kStageW;
+  if (p.w_stages > 8) p.w_stages = 8;
+  const size_t smem = static_cast<size_t>(p.x_stages) * p.x_boxes * p.m_pad * 128 + static_cast<size_t>(p.w_stages) * kStageW + kBars + 1024;
+  ensure_dynamic_smem(gemm_unpack_kernel<T>, smem);
+  const long long units = static_cast<long long>((p.N + kTileN - 1) / kTileN) * (p.K / kSuper);
+  const int sms = sm_count();
+  launch_kernel(gemm_unpack_kernel<T>, dim3(static_cast<unsigned>(units < sms ? units : sms)), dim3(kUnpackThreads), smem, stream,
+                /*pdl=*/true, /*cooperative=*/false, tmW, tmX, p);
+}
+
+}  // namespace
+
+int gemm_unpack_box(int q_type) {
+  return q_type == kQ_Q4_K ? Super<kQ_Q4_K>::kBox : (q_type == kQ_Q5_K ? Super<kQ_Q5_K>::kBox : (q_type == kQ_Q6_K ? Super<kQ_Q6_K>::kBox : 0));
+}
+
+void launch_gemm_unpack(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmUnpackParams& p, int q_type, cudaStream_t stream) {
+  if (q_type == kQ_Q4_K) launch_type<kQ_Q4_K>(tmW, tmX, p, stream);
+  else if (q_type == kQ_Q5_K) launch_type<kQ_Q5_K>(tmW, tmX, p, stream);
+  else launch_type<kQ_Q6_K>(tmW, tmX, p, stream);
+}
+
+}  // namespace oxb

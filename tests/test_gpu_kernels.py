@@ -787,6 +787,37 @@ def test_gemm_with_gguf_weights_unpacked_in_the_kernel(ops, qname):
     assert _rel_err(out, x.float() @ wd.T + bias.float()) < 1e-2
 
 
+@pytest.mark.parametrize("qname", ["Q4_K", "Q5_K", "Q6_K"])
+@pytest.mark.parametrize("m,n,k", [(1, 128, 2048), (9, 200, 2048), (16, 1, 4096), (33, 8200, 2048), (64, 130, 14336), (65, 384, 2048), (128, 640, 4096),
+                                   (129, 136, 2048), (200, 1000, 2048), (256, 20000, 2048)])
+def test_gemm_with_super_blocks_unpacked_into_tmem(ops, qname, m, n, k):
+    """Every row count class, ragged tiles, runs of units that begin and end inside a row of units, a view with a row stride, and
+    results added to what is there: against fp32 of the decoded weights rounded to bf16 (the sums' order alone differs)."""
+    from oxide_tech_llm_engine_b200.formats import quants
+    from oxide_tech_llm_engine_b200.models.llama import random_quant_linear
+
+    gen = torch.Generator(device=DEV).manual_seed(n + m)
+    code = quants.TYPES[qname].code
+    if qname == "Q5_K":
+        raw = quants.quantize_2d(qname, torch.randn(min(n, 256), k, generator=torch.Generator().manual_seed(n)).numpy() * 0.05)
+        w_dev = torch.from_numpy(raw).to(DEV).view(min(n, 256), -1).repeat(-(-n // 256), 1)[:n].reshape(-1).contiguous()
+    else:
+        w_dev = random_quant_linear(qname, n, k, torch.device(DEV), gen).w
+    wide = torch.randn(m, k + 64, device=DEV, generator=gen).to(torch.bfloat16)
+    x = wide[:, 64:]
+    wd = torch.empty(n, k, dtype=torch.bfloat16, device=DEV)
+    ops.dequant_rows(code, w_dev, wd, n_src_rows=n, k=k)
+    out = torch.full((m, n + 3), 0.5, device=DEV)
+    ops.gemm_packed(x, code, w_dev, n, out[:, :n], epi=ops.EPI_RED_F32)
+    torch.cuda.synchronize()
+    ops.check_status()
+    ref = x.double() @ wd.double().T + 0.5
+    # 32-bit sums of k products in another order, and weights that another formula may round to the neighbouring bf16
+    assert ((out[:, :n] - ref).norm() / ref.norm()).item() < 2e-4
+    assert _rel_err(out[:, :n], ref) < 2e-3
+    assert (out[:, n:] == 0.5).all()
+
+
 def test_norm_and_swiglu_write_the_int8_view_of_their_output(ops):
     """finalize_norm and swiglu with `q8`: the int8 blocks, scales and sums are exactly what the
     stand-alone quantiser makes of the bf16 rows those kernels wrote."""
