@@ -151,64 +151,69 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     } else if (warp == 1) {
       // ------------------------------ MMA issuer --------------------------------
-      if (lane == 0) {
-        constexpr uint32_t idesc_s = make_idesc(kFmtBF16, kFmtBF16, BQ, BKV);
-        constexpr uint32_t idesc_o = make_idesc(kFmtBF16, kFmtBF16, BQ, D, 0, 1);  // V is MN-major
-        bool ok = mbar_wait(q_full, 0);
-        auto issue_s = [&](int g, uint32_t k_item) {
-          const uint32_t qa = smem_u32(sQ) + g * L::kSlotBytes;
-          const uint32_t kb = smem_u32(ring) + (k_item % NS) * L::kSlotBytes;
-  #pragma unroll
+      // the whole warp walks and waits, an elected lane issues (elect_one: the operands stay in uniform registers)
+      constexpr uint32_t idesc_s = make_idesc(kFmtBF16, kFmtBF16, BQ, BKV);
+      constexpr uint32_t idesc_o = make_idesc(kFmtBF16, kFmtBF16, BQ, D, 0, 1);  // V is MN-major
+      bool ok = mbar_wait(q_full, 0);
+      auto issue_s = [&](int g, uint32_t k_item, bool last) {
+        const uint32_t qa = smem_u32(sQ) + g * L::kSlotBytes;
+        const uint32_t kb = smem_u32(ring) + (k_item % NS) * L::kSlotBytes;
+        if (elect_one()) {
+#pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t at = (kk >> 2) * kHalfBytes + (kk & 3) * 32;
             tc_mma_f16(tmem_base + g * 128, make_desc_kmajor_sw128(qa + at), make_desc_kmajor_sw128(kb + at), idesc_s,
                        kk != 0 ? 1u : 0u);
           }
           tc_commit(&s_full[g]);
-        };
-        if (ok && n_tiles > 0) {
-          ok = mbar_wait(&full[0], 0);
-          tc_fence_after_sync();
-          if (ok) {
-            issue_s(0, 0);
-            issue_s(1, 0);
-            tc_commit(&empty[0]);
-          }
+          if (last) tc_commit(&empty[k_item % NS]);
         }
-        for (int j = 0; j < n_tiles && ok; ++j) {
-          const uint32_t v_item = 2 * j + 1, k_item = 2 * j + 2;
-          ok = mbar_wait(&full[v_item % NS], (v_item / NS) & 1);
-          for (int g = 0; g < 2 && ok; ++g) {
-            if (!mbar_wait(&p_full[g], j & 1)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after_sync();
-            const uint32_t vb = smem_u32(ring) + (v_item % NS) * L::kSlotBytes;
-            const uint32_t pa = tmem_base + g * 128, od = tmem_base + 256 + g * D;
-  #pragma unroll
+        __syncwarp();
+      };
+      if (n_tiles > 0) {
+        ok = ok && mbar_wait(&full[0], 0);
+        ok = __all_sync(0xffffffffu, ok);
+        tc_fence_after_sync();
+        if (ok) {
+          issue_s(0, 0, false);
+          issue_s(1, 0, true);
+        }
+      }
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        const uint32_t v_item = 2 * j + 1, k_item = 2 * j + 2;
+        ok = mbar_wait(&full[v_item % NS], (v_item / NS) & 1);
+        for (int g = 0; g < 2; ++g) {
+          if (ok && !mbar_wait(&p_full[g], j & 1)) ok = false;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after_sync();
+          const uint32_t vb = smem_u32(ring) + (v_item % NS) * L::kSlotBytes;
+          const uint32_t pa = tmem_base + g * 128, od = tmem_base + 256 + g * D;
+          if (elect_one()) {
+#pragma unroll
             for (int kk = 0; kk < BKV / 16; ++kk)
               tc_mma_f16_ts(od, pa + kk * 8, make_desc_mnmajor_sw128(vb + kk * 2048, kHalfBytes, 1024), idesc_o,
                             (j | kk) != 0 ? 1u : 0u);
             if constexpr (EXACT) {
-  #pragma unroll
+#pragma unroll
               for (int kk = 0; kk < BKV / 16; ++kk)
                 tc_mma_f16_ts(od, pa + 64 + kk * 8, make_desc_mnmajor_sw128(vb + kk * 2048, kHalfBytes, 1024), idesc_o, 1u);
             }
             if (g == 1) tc_commit(&empty[v_item % NS]);
-            if (j + 1 < n_tiles) {
-              if (g == 0) ok = mbar_wait(&full[k_item % NS], (k_item / NS) & 1);
-              if (!ok) break;
-              tc_fence_after_sync();
-              issue_s(g, k_item);
-              if (g == 1) tc_commit(&empty[k_item % NS]);
-            } else {
-              tc_commit(&o_full[g]);
-            }
+            if (j + 1 == n_tiles) tc_commit(&o_full[g]);
           }
+          __syncwarp();
+          if (j + 1 == n_tiles) continue;
+          if (g == 0) {
+            ok = mbar_wait(&full[k_item % NS], (k_item / NS) & 1);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after_sync();
+          }
+          issue_s(g, k_item, g == 1);
         }
-        if (!ok) set_status_once(status, kStatusMbarTimeoutMma);
       }
+      if (!ok && lane == 0) set_status_once(status, kStatusMbarTimeoutMma);
     }
   } else {
     warpgroup_regs_inc<kSoftmaxRegs>();

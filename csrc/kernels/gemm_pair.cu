@@ -149,31 +149,36 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (lane == 0) pdl_launch_dependents();  // every operand of this CTA has been requested
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (even CTA) ---------------------
-    if (rank == 0 && lane == 0) {
+    // the whole warp walks and waits, an elected lane issues (elect_one: the operands stay in uniform registers)
+    if (rank == 0) {
       constexpr uint32_t idesc = make_idesc(kFmtBF16, kFmtBF16, kTile, kTile);
-      uint32_t iter = 0, t = 0;
+      uint32_t s = 0, phase = 0, t = 0;
       bool ok = true;
       for (int w = first; w < n_work && ok; w += step, ++t) {
         const uint32_t buf = t & 1, use = t >> 1;
         if (use >= 1 && !mbar_wait_cluster(&tmem_empty[buf], (use & 1) ^ 1, spin)) ok = false;
-        tc_fence_after_sync();
-        for (int kb = 0; kb < total_kb && ok; ++kb, ++iter) {
-          const int s = iter % kStages;
-          if (!mbar_wait_cluster(&full[s], (iter / kStages) & 1, spin)) {
-            ok = false;
-            break;
-          }
+        for (int kb = 0; kb < total_kb; ++kb) {
+          if (ok && !mbar_wait_cluster(&full[s], phase, spin)) ok = false;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
           tc_fence_after_sync();
           const uint32_t a = smem_u32(smem + s * 2 * kOpBytes), b = a + kOpBytes;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k)
-            tc_mma_f16_pair(tmem_base + buf * kTile, make_desc_kmajor_sw128(a + k * 32), make_desc_kmajor_sw128(b + k * 32),
-                            idesc, (kb | k) != 0 ? 1u : 0u);
-          tc_commit_pair(&empty[s]);
+            for (int k = 0; k < kBK / 16; ++k)
+              tc_mma_f16_pair(tmem_base + buf * kTile, make_desc_kmajor_sw128(a + k * 32), make_desc_kmajor_sw128(b + k * 32),
+                              idesc, (kb | k) != 0 ? 1u : 0u);
+            tc_commit_pair(&empty[s]);
+            if (kb == total_kb - 1) tc_commit_pair(&tmem_full[buf]);
+          }
+          __syncwarp();
+          if (++s == kStages) {
+            s = 0;
+            phase ^= 1;
+          }
         }
-        if (ok) tc_commit_pair(&tmem_full[buf]);
       }
-      if (!ok) set_status_once(p.status, kStatusMbarTimeoutMma);
+      if (!ok && lane == 0) set_status_once(p.status, kStatusMbarTimeoutMma);
     }
   } else {
     // ------------------------------ epilogue ----------------------------------
