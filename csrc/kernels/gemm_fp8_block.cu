@@ -2,12 +2,19 @@
 //
 //   C[m, n] = sum_kb  sa[m, kb] * sw[n / 128, kb] * sum_{k in block kb} A8[m, k] * W8[n, k]
 //
-// One CTA computes a 128 x 128 output tile. K advances in blocks of 128 fp8 values (128 bytes =
+// A cluster of CTAs computes a 128 x 128 output tile, each CTA a run of its K blocks of 128 fp8 values (128 bytes =
 // one swizzle atom row). Every K block is one fresh accumulation (`kind::f8f6f4`, four K=32
-// instructions) into one of two TMEM buffers; the four epilogue warps read that buffer back,
+// instructions) into one of two TMEM buffers; eight epilogue warps read that buffer back,
 // multiply by the two scales of the block and add into fp32 registers (the "promotion" that keeps
 // the scales outside the tensor core), while the MMA warp already fills the other buffer.
+// At the end the CTAs of a cluster exchange their sums through distributed shared memory and each stores a share of the columns.
 // Warp 0 feeds a TMA ring, warp 1 issues the MMAs; every wait is bounded.
+//
+// What bounds it: with few rows the weights from HBM (57344 x 8192: 64 rows 107 us, 4.4 TB/s; 8192 x 28672 with 128 rows 68 us), with
+// many the promotion, as long as the operands of a block take through shared memory (4096 rows: 2036 and 988 us, 1890 and 1947
+// TFLOP/s). One CTA per tile and SM, and four warps whose every read of an accumulator waited for itself and for its
+// scales, took 183 and 163 us with 128 rows, 3604 and 2227 us with 4096. Two CTAs per SM (96 registers, three stages) hide each
+// other's start, waits and stores.
 //
 // Reference counterpart: the e4m3 codec and the scaled fp8 block of crates/oxide-quant/src/fp8.rs
 // (Fp8E4M3 :13-98, BlockFp8E4M3 quantize / dequantize / dot_product :185-245). The reference has no
@@ -25,15 +32,32 @@ namespace oxb {
 namespace {
 
 constexpr int BM = 128, BN = 128, BKB = 128;  // BKB: bytes = fp8 elements per K block
-constexpr int STAGES = 5;
+constexpr int STAGES = 3;
 constexpr int kTileBytes = 128 * BKB;  // A tile = B tile = 16 KB
-constexpr int kThreads = 192;
+constexpr int kEpiWarps = 8;           // two per TMEM lane quarter, 64 columns each
+constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kBarOffset = STAGES * 2 * kTileBytes;
 constexpr int kSmemTotal = kBarOffset + 256 + 1024;
+static_assert(BM * BN * 4 <= kBarOffset, "the ring holds a tile's sums when it is idle");
 
-__global__ void __launch_bounds__(kThreads, 1)
+// 8 columns of a row -> bias, bf16, their place.
+__device__ __forceinline__ void store_cols(const Fp8GemmParams& p, __nv_bfloat16* d, bool vec, int col, const float (&v)[8]) {
+  float o[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) o[e] = p.bias != nullptr && col + e < p.N ? v[e] + __bfloat162float(p.bias[col + e]) : v[e];
+  if (vec && col + 8 <= p.N) {
+    *reinterpret_cast<uint4*>(d + col) =
+        make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (col + e < p.N) d[col + e] = __float2bfloat16(o[e]);
+  }
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const Fp8GemmParams p) {
+                      const Fp8GemmParams p, const int split) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem =
       reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -46,8 +70,12 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  const int n_kb = (p.K + BKB - 1) / BKB;
+  const int z = static_cast<int>(blockIdx.x) % split;  // place in the cluster
+  const int m0 = static_cast<int>(blockIdx.x) / split * BM, n0 = blockIdx.y * BN;
+  const int all_kb = (p.K + BKB - 1) / BKB;
+  const int per = (all_kb + split - 1) / split;
+  const int kb0 = z * per;
+  const int n_kb = all_kb - kb0 < per ? all_kb - kb0 : per;  // may be none
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
@@ -58,8 +86,8 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
     mbar_init(&tmem_full[0], 1);
     mbar_init(&tmem_full[1], 1);
-    mbar_init(&tmem_empty[0], 4);
-    mbar_init(&tmem_empty[1], 4);
+    mbar_init(&tmem_empty[0], kEpiWarps);
+    mbar_init(&tmem_empty[1], kEpiWarps);
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -71,36 +99,51 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
+  const int q = warp & 3, half = (warp - 2) >> 2;  // epilogue: lane quarter, 64 columns
+  const int row = m0 + q * 32 + lane;
+  const bool row_ok = row < p.M;
+  float acc[64];
+#pragma unroll
+  for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+  bool ok = true;
+
   if (warp == 0) {
-    if (lane == 0) {
-      for (int kb = 0; kb < n_kb; ++kb) {
-        const int s = kb % STAGES;
-        if (kb >= STAGES && !mbar_wait(&empty[s], ((kb / STAGES) & 1) ^ 1)) {
-          set_status_once(p.status, kStatusMbarTimeoutProducer);
-          break;
-        }
-        mbar_arrive_expect_tx(&full[s], 2 * kTileBytes);
-        tma_load_2d(sB + s * kTileBytes, &tmB, &full[s], kb * BKB, n0);
-        tma_load_2d(sA + s * kTileBytes, &tmA, &full[s], kb * BKB, m0);
+    int s = 0;
+    uint32_t ph = 1;
+    for (int kb = 0; kb < n_kb; ++kb) {
+      if (kb >= STAGES && !mbar_wait(&empty[s], ph)) ok = false;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutProducer);
+        break;
+      }
+      if (lane == 0) mbar_arrive_expect_tx(&full[s], 2 * kTileBytes);
+      __syncwarp();
+      // copies that one thread issues complete one after the other: a lane for each copy of the ring
+      if (lane == 2 * s) tma_load_2d(sB + s * kTileBytes, &tmB, &full[s], (kb0 + kb) * BKB, n0);
+      if (lane == 2 * s + 1) tma_load_2d(sA + s * kTileBytes, &tmA, &full[s], (kb0 + kb) * BKB, m0);
+      if (++s == STAGES) {
+        s = 0;
+        ph ^= 1;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(kFmtE4M3, kFmtE4M3, BM, BN);
-      for (int kb = 0; kb < n_kb; ++kb) {
-        const int s = kb % STAGES;
-        const uint32_t buf = kb & 1;
-        if (kb >= 2 && !mbar_wait(&tmem_empty[buf], ((kb >> 1) & 1) ^ 1)) {
-          set_status_once(p.status, kStatusMbarTimeoutMma);
-          break;
-        }
-        if (!mbar_wait(&full[s], (kb / STAGES) & 1)) {
-          set_status_once(p.status, kStatusMbarTimeoutMma);
-          break;
-        }
-        tc_fence_after_sync();
-        const uint32_t a_addr = smem_u32(sA + s * kTileBytes);
-        const uint32_t b_addr = smem_u32(sB + s * kTileBytes);
+    constexpr uint32_t idesc = make_idesc(kFmtE4M3, kFmtE4M3, BM, BN);
+    int s = 0;
+    uint32_t ph = 0;
+    for (int kb = 0; kb < n_kb; ++kb) {
+      const uint32_t buf = kb & 1;
+      if (kb >= 2 && !mbar_wait(&tmem_empty[buf], ((kb >> 1) & 1) ^ 1)) ok = false;
+      if (ok && !mbar_wait(&full[s], ph)) ok = false;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutMma);
+        break;
+      }
+      tc_fence_after_sync();
+      const uint32_t a_addr = smem_u32(sA + s * kTileBytes);
+      const uint32_t b_addr = smem_u32(sB + s * kTileBytes);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < BKB / 32; ++k)
           tc_mma_f8(tmem_base + buf * BN, make_desc_kmajor_sw128(a_addr + k * 32),
@@ -108,99 +151,121 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         tc_commit(&empty[s]);
         tc_commit(&tmem_full[buf]);
       }
+      __syncwarp();
+      if (++s == STAGES) {
+        s = 0;
+        ph ^= 1;
+      }
     }
   } else {
-    const int q = warp & 3;
-    const int row = m0 + q * 32 + lane;
-    const bool row_ok = row < p.M;
-    const int kb_cols = n_kb;
-    const float* sw_row = p.sw + static_cast<long long>(blockIdx.y) * kb_cols;
-    float acc[BN];
-#pragma unroll
-    for (int j = 0; j < BN; ++j) acc[j] = 0.f;
-    bool ok = true;
+    const bool live = m0 + q * 32 < p.M;  // a quarter without rows has nothing to add up
+    const float* sw_row = p.sw + static_cast<long long>(blockIdx.y) * all_kb + kb0;
+    const float* sa_row = p.sa_t + static_cast<long long>(kb0) * p.sa_ld + (row_ok ? row : 0);
+    // the scales of a block are requested one block ahead
+    float sa = n_kb > 0 ? __ldg(sa_row) : 0.f, sw = n_kb > 0 ? __ldg(sw_row) : 0.f;
     for (int kb = 0; kb < n_kb; ++kb) {
       const uint32_t buf = kb & 1;
-      if (ok && !mbar_wait(&tmem_full[buf], (kb >> 1) & 1)) {
-        if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutEpilogue);
-        ok = false;
+      const float sc = sa * sw;
+      if (kb + 1 < n_kb) {
+        sa = __ldg(sa_row + static_cast<long long>(kb + 1) * p.sa_ld);
+        sw = __ldg(sw_row + kb + 1);
       }
+      if (!mbar_wait(&tmem_full[buf], (kb >> 1) & 1)) ok = false;
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      if (!ok) {
+        if (lane == 0) set_status_once(p.status, kStatusMbarTimeoutEpilogue);
+        break;
+      }
       tc_fence_after_sync();
-      const float sc = (row_ok ? __ldg(p.sa_t + static_cast<long long>(kb) * p.sa_ld + row) : 0.f) *
-                       __ldg(sw_row + kb);
-      const uint32_t lane_addr = tmem_base + buf * BN + (static_cast<uint32_t>(q * 32) << 16);
+      if (live) {
+        const uint32_t at = tmem_base + buf * BN + half * 64 + (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(lane_addr + c * 32, r);
-        tmem_ld_wait();
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[16];
+          tmem_ld_32x32b_x16(at + c * 16, r);
+          tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[c * 32 + j] = fmaf(__uint_as_float(r[j]), sc, acc[c * 32 + j]);
+          for (int j = 0; j < 16; ++j) acc[c * 16 + j] = fmaf(__uint_as_float(r[j]), sc, acc[c * 16 + j]);
+        }
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[buf]);
     }
-    if (ok && row_ok) {
-      __nv_bfloat16* d = p.C + static_cast<long long>(row) * p.ldc + n0;
-      long long ld = p.ldc;
-      if (p.n_owners > 0) {
-        int owner = row / p.rows_per_owner;
-        if (owner >= p.n_owners) owner = p.n_owners - 1;
-        __nv_bfloat16* base = nullptr;
+  }
+
+  // where a row goes: C, or the receive slab of the rank that owns it
+  auto row_ptr = [&](int r) -> __nv_bfloat16* {
+    if (p.n_owners <= 0) return p.C + static_cast<long long>(r) * p.ldc;
+    int owner = r / p.rows_per_owner;
+    if (owner >= p.n_owners) owner = p.n_owners - 1;
+    __nv_bfloat16* base = nullptr;
 #pragma unroll
-        for (int o = 0; o < 8; ++o)
-          if (o == owner) base = p.slab[o];
-        d = base + (static_cast<long long>(p.my_rank) * p.rows_per_owner + (row - owner * p.rows_per_owner)) * p.slab_ld + n0;
-        ld = p.slab_ld;
-      }
-      const bool vec = (ld & 7) == 0 && n0 + BN <= p.N;
+    for (int o = 0; o < 8; ++o)
+      if (o == owner) base = p.slab[o];
+    return base + (static_cast<long long>(p.my_rank) * p.rows_per_owner + (r - owner * p.rows_per_owner)) * p.slab_ld;
+  };
+  const bool vec = ((p.n_owners > 0 ? p.slab_ld : p.ldc) & 7) == 0;
+  if (split == 1) {
+    if (warp >= 2 && ok && row_ok) {
+      __nv_bfloat16* d = row_ptr(row);
 #pragma unroll
-      for (int j = 0; j < BN; j += 8) {
-        float v[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          v[e] = acc[j + e];
-          if (p.bias != nullptr && n0 + j + e < p.N) v[e] += __bfloat162float(p.bias[n0 + j + e]);
-        }
-        if (vec) {
-          uint4 o4;
-          o4.x = pack_bf16x2(v[0], v[1]);
-          o4.y = pack_bf16x2(v[2], v[3]);
-          o4.z = pack_bf16x2(v[4], v[5]);
-          o4.w = pack_bf16x2(v[6], v[7]);
-          *reinterpret_cast<uint4*>(d + j) = o4;
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e)
-            if (n0 + j + e < p.N) d[j + e] = __float2bfloat16(v[e]);
-        }
+      for (int j = 0; j < 64; j += 8) {
+        const float v[8] = {acc[j], acc[j + 1], acc[j + 2], acc[j + 3], acc[j + 4], acc[j + 5], acc[j + 6], acc[j + 7]};
+        store_cols(p, d, vec, n0 + half * 64 + j, v);
       }
     }
-    tc_fence_before_sync();
-    if (p.done_ticket != nullptr) {
-      // one system-scope fence per CTA after the barrier, then the grid-wide ticket; the last CTA
-      // signals every owner with relaxed adds (see the bf16 GEMM for the reasoning)
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (warp == 2 && lane == 0) {
-        __threadfence_system();
-        const uint32_t total = gridDim.x * gridDim.y;
-        const uint32_t old = atomicAdd(p.done_ticket, 1u);
-        if (old == total - 1) {
-          *p.done_ticket = 0;
-          __threadfence_system();
+  } else {
+    // sums of 8 columns: [16 groups][128 rows][8] in the ring, which is idle now (the last product has been read back)
+    float* part = reinterpret_cast<float*>(smem);
+    if (warp >= 2) {
 #pragma unroll
-          for (int o = 0; o < 8; ++o)
-            if (o < p.n_owners && p.arrive[o] != nullptr)
-              asm volatile("red.relaxed.sys.global.add.u32 [%0], %1;" ::"l"(p.arrive[o]), "r"(1u) : "memory");
+      for (int g = 0; g < 8; ++g) {
+        float4* to = reinterpret_cast<float4*>(part + ((half * 8 + g) * 128 + q * 32 + lane) * 8);
+        to[0] = make_float4(acc[8 * g], acc[8 * g + 1], acc[8 * g + 2], acc[8 * g + 3]);
+        to[1] = make_float4(acc[8 * g + 4], acc[8 * g + 5], acc[8 * g + 6], acc[8 * g + 7]);
+      }
+    }
+    cluster_sync_all();
+    if (warp >= 2) {
+      const int t = threadIdx.x - 64, r = t & 127;
+      __nv_bfloat16* d = m0 + r < p.M ? row_ptr(m0 + r) : nullptr;
+      for (int g = z + split * (t >> 7); g < 16; g += 2 * split) {
+        if (d == nullptr) break;
+        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int c = 0; c < split; ++c) {
+          const uint32_t from = cluster_addr(part + (g * 128 + r) * 8, c);
+          float4 x, y;
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(from));
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w) : "r"(from + 16));
+          v[0] += x.x, v[1] += x.y, v[2] += x.z, v[3] += x.w, v[4] += y.x, v[5] += y.y, v[6] += y.z, v[7] += y.w;
         }
+        store_cols(p, d, vec, n0 + g * 8, v);
+      }
+    }
+  }
+  if (warp >= 2 && p.done_ticket != nullptr) {
+    // one system-scope fence per CTA after the barrier, then the grid-wide ticket; the last CTA
+    // signals every owner with relaxed adds (see the bf16 GEMM for the reasoning)
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+    if (warp == 2 && lane == 0) {
+      __threadfence_system();
+      const uint32_t total = gridDim.x * gridDim.y;
+      const uint32_t old = atomicAdd(p.done_ticket, 1u);
+      if (old == total - 1) {
+        *p.done_ticket = 0;
+        __threadfence_system();
+#pragma unroll
+        for (int o = 0; o < 8; ++o)
+          if (o < p.n_owners && p.arrive[o] != nullptr)
+            asm volatile("red.relaxed.sys.global.add.u32 [%0], %1;" ::"l"(p.arrive[o]), "r"(1u) : "memory");
       }
     }
   }
 
+  tc_fence_before_sync();
   __syncthreads();
+  if (split > 1) cluster_sync_all();  // the sums of this CTA have been read
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 2 * BN);
@@ -288,8 +353,32 @@ __global__ void quant_act_fp8_kernel(const __nv_bfloat16* x, long long x_ld, uin
 void launch_gemm_fp8_block(const CUtensorMap& tmA, const CUtensorMap& tmB, const Fp8GemmParams& p,
                            cudaStream_t stream) {
   ensure_dynamic_smem(gemm_fp8_block_kernel, kSmemTotal);
-  dim3 grid((p.M + BM - 1) / BM, (p.N + BN - 1) / BN);
-  gemm_fp8_block_kernel<<<grid, kThreads, kSmemTotal, stream>>>(tmA, tmB, p);
+  const int m_tiles = (p.M + BM - 1) / BM, n_tiles = (p.N + BN - 1) / BN, n_kb = (p.K + BKB - 1) / BKB;
+  // CTAs per tile: the fewest rounds of two CTAs per SM times the K blocks of one, and the start and the exchange of a CTA, which
+  // take about as long as 6 blocks
+  int split = 1;
+  long long best = 0;
+  for (int s = 1; s <= 8 && (s == 1 || n_kb >= 8 * s); ++s) {
+    const long long rounds = (static_cast<long long>(m_tiles) * n_tiles * s + 2 * sm_count() - 1) / (2 * sm_count());
+    const long long cost = rounds * ((n_kb + s - 1) / s + 6);
+    if (s == 1 || cost < best) {
+      best = cost;
+      split = s;
+    }
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(m_tiles * split, n_tiles);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmemTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, gemm_fp8_block_kernel, tmA, tmB, p, split);
 }
 
 void launch_quant_act_fp8(const __nv_bfloat16* x, long long x_ld, uint8_t* q, long long q_ld,

@@ -1091,6 +1091,26 @@ def test_gemm_fp8_block_scaled(ops, M, N, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(1, 128, 28672), (117, 1000, 8192), (33, 10240, 8192), (129, 8192, 8080), (256, 1, 1024), (31, 57344, 1024), (700, 2568, 3072)])
+def test_gemm_fp8_block_scaled_over_clusters(ops, M, N, K):
+    """K shared out over 1 to 8 CTAs of a cluster, ragged in every direction, against 64 bits: bf16 rounding of the results (2^-9 at most) and
+    nothing else of that size."""
+    gen = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x = (torch.randn(M, K, device=DEV, generator=gen) * 2).to(torch.bfloat16)
+    w8, sw = ops.quant_weight_fp8_block(torch.randn(N, K, device=DEV, generator=gen) * 0.05)
+    a8, sa_t = ops.quant_act_fp8(x)
+    out = torch.full((M, N + 8), 7.0, device=DEV).to(torch.bfloat16)
+    ops.gemm_fp8_block(a8, sa_t, w8, sw, out=out[:, :N])
+    torch.cuda.synchronize()
+    ops.check_status()
+    a = a8.double() * sa_t[:, :M].t().double().repeat_interleave(128, 1)[:, :K]
+    w = w8.double() * sw.double().repeat_interleave(128, 0)[:N].repeat_interleave(128, 1)[:, :K]
+    ref = a @ w.t()
+    assert ((out[:, :N].double() - ref).norm() / ref.norm()).item() < 2.0 ** -9
+    assert (out[:, N:] == 7.0).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("bn", [64, 128, 256])
 @pytest.mark.parametrize("m,n,k", [(200, 512, 256), (256, 1280, 1024), (8, 768, 192)])
 def test_gemm_tile_major_weights(ops, m, n, k, bn):
