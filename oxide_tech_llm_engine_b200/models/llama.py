@@ -608,13 +608,16 @@ class DeviceModel(GemmShapes):
         return 4 if getattr(lin, "dense", None) is not None else 8
 
     def _qlinear(self, lin: QuantLinear, x: torch.Tensor, out_f32: torch.Tensor, ld_out: Optional[int] = None,
-                 xq=None):
-        """out_f32[:, :n] = x @ W^T for a packed weight: MMVQ for small batches, else dequant + tcgen05."""
+                 xq=None, zeroed: bool = False):
+        """out_f32[:, :n] = x @ W^T for a packed weight: MMVQ for small batches, else dequant + tcgen05. `zeroed`: the rows are
+        zero already (the accumulators that their readers clear), so a kernel that adds needs no clearing launch."""
         m = x.shape[0]
         if lin.packed and m <= self._mmvq_rows(lin):
             ops.mmvq(lin.code, lin.w, x, out_f32, n=lin.n, k=lin.k,
                      xq=xq if lin.code in ops.INT8_MMVQ_CODES else None)
             return
+        if not zeroed:
+            out_f32[:m].zero_() if out_f32.is_contiguous() else out_f32[:m].fill_(0)
         w = lin.w
         if lin.packed and getattr(lin, "dense", None) is not None:
             w = lin.dense
@@ -626,14 +629,12 @@ class DeviceModel(GemmShapes):
             # the unpacking is the bound: spread it over as many SMs as the tiles and K allow
             tiles = (lin.n + 127) // 128
             sp = max(1, min(self._sms // tiles, lin.k // 256, 16))
-            out_f32[:m].zero_() if out_f32.is_contiguous() else out_f32[:m].fill_(0)
             ops.gemm_packed(x, lin.code, lin.w, lin.n, out_f32[:m], epi=ops.EPI_RED_F32, mt=mt, splits=sp)
             return
         elif lin.packed:
             w = self._scratch_for(lin.n, lin.k)
             ops.dequant_rows(lin.code, lin.w, w, n_src_rows=lin.n, k=lin.k)
         bn = ops.pick_bn(lin.n, (m + 127) // 128, can_split=True)
-        out_f32[:m].zero_() if out_f32.is_contiguous() else out_f32[:m].fill_(0)
         ops.gemm(x, w, epi=ops.EPI_RED_F32, dst_ptrs=[out_f32.data_ptr()], bn=bn,
                  splits=ops.pick_splits(m, lin.n, lin.k, bn), dst_ld=out_f32.stride(0))
 
@@ -809,13 +810,13 @@ class DeviceModel(GemmShapes):
         for li, L in enumerate(self.layers):
             xq = xq_d if xq_d is not None else self._q8(g0)
             if "attn_qkv" in L:
-                self._qlinear(L["attn_qkv"], g0, self.qkv_acc[:M], xq=xq)
+                self._qlinear(L["attn_qkv"], g0, self.qkv_acc[:M], xq=xq, zeroed=True)
             elif xq is not None and L.get("qkv_mix") is not None and M <= self._mmvq_rows(L["attn_q"]):
                 ops.mmvq_mixed(L["qkv_mix"], g0, self.qkv_acc[:M], k=d, xq=xq)
             else:
-                self._qlinear(L["attn_q"], g0, self.qkv_acc[:M, :qd], xq=xq)
-                self._qlinear(L["attn_k"], g0, self.qkv_acc[:M, qd:qd + kd], xq=xq)
-                self._qlinear(L["attn_v"], g0, self.qkv_acc[:M, qd + kd:], xq=xq)
+                self._qlinear(L["attn_q"], g0, self.qkv_acc[:M, :qd], xq=xq, zeroed=True)
+                self._qlinear(L["attn_k"], g0, self.qkv_acc[:M, qd:qd + kd], xq=xq, zeroed=True)
+                self._qlinear(L["attn_v"], g0, self.qkv_acc[:M, qd + kd:], xq=xq, zeroed=True)
             ops.qkv_rope_append(acc_f32=self.qkv_acc, bias=L["b_qkv"], q_norm_w=L["q_norm"], k_norm_w=L["k_norm"],
                                 norm_eps=1e-6, norm_w_offset=cfg.norm_weight_offset, positions=s.positions,
                                 slot_mapping=s.slot_mapping, inv_freq=self.inv_freq, rope_mscale=self.rope_mscale,
@@ -825,19 +826,19 @@ class DeviceModel(GemmShapes):
             xq_o = self._q8_views(M, cfg.q_dim) if (s.n_prefill == 0 and s.n_decode == M) else None
             self._attention(s, li, q8=xq_o)
             self._qlinear(L["attn_output"], self.attn_out[:M], acc0[:M],
-                          xq=xq_o if xq_o is not None else self._q8(self.attn_out[:M]))
+                          xq=xq_o if xq_o is not None else self._q8(self.attn_out[:M]), zeroed=True)
             self._finalize(M, L["ffn_norm"], acc=0, gather="gather1", flag_base=F_AG1, r0=0, q8=xq_d)
             xq = xq_d if xq_d is not None else self._q8(g1)
             if "ffn_gate_up" in L:
-                self._qlinear(L["ffn_gate_up"], g1, self.gu_acc[:M], xq=xq)
+                self._qlinear(L["ffn_gate_up"], g1, self.gu_acc[:M], xq=xq, zeroed=True)
             elif xq is not None and L.get("gu_mix") is not None and M <= self._mmvq_rows(L["ffn_gate"]):
                 ops.mmvq_mixed(L["gu_mix"], g1, self.gu_acc[:M], k=d, xq=xq)
             else:
-                self._qlinear(L["ffn_gate"], g1, self.gu_acc[:M, :self.i_l], xq=xq)
-                self._qlinear(L["ffn_up"], g1, self.gu_acc[:M, self.i_l:], xq=xq)
+                self._qlinear(L["ffn_gate"], g1, self.gu_acc[:M, :self.i_l], xq=xq, zeroed=True)
+                self._qlinear(L["ffn_up"], g1, self.gu_acc[:M, self.i_l:], xq=xq, zeroed=True)
             xq_a = self._q8_views(M, self.i_l)
             ops.swiglu(acc_f32=self.gu_acc, out=self.act, m=M, i=self.i_l, act=self._act_code, q8=xq_a)
-            self._qlinear(L["ffn_down"], self.act[:M], acc1[:M], xq=xq_a if xq_a is not None else self._q8(self.act[:M]))
+            self._qlinear(L["ffn_down"], self.act[:M], acc1[:M], xq=xq_a if xq_a is not None else self._q8(self.act[:M]), zeroed=True)
             if li != cfg.n_layers - 1:
                 self._finalize(M, self.layers[li + 1]["attn_norm"], acc=1, gather="gather0", flag_base=F_AG0, r0=0,
                                q8=xq_d)
@@ -1005,6 +1006,8 @@ class DeviceModel(GemmShapes):
         for name in ("acc0", "acc1"):
             self.ws.local(name).zero_()
         self.qkv_acc.zero_()
+        if self.weight_mode == "quant":
+            self.gu_acc.zero_()
         torch.cuda.synchronize(self.device)
 
     def close(self) -> None:
