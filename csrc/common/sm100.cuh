@@ -59,6 +59,14 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Asks L2 for the bytes [p, p + bytes) of global memory (the whole 16-byte units among them); changes nothing else.
+__device__ __forceinline__ void l2_prefetch(const void* p, long long bytes) {
+  const uintptr_t lo = (reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15);
+  const uintptr_t hi = (reinterpret_cast<uintptr_t>(p) + static_cast<uintptr_t>(bytes)) & ~uintptr_t(15);
+  if (hi > lo)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"(static_cast<uint32_t>(hi - lo)) : "memory");
+}
+
 // True in one lane of a converged warp, the same one each time. What that lane then does alone is known to come from one thread: the
 // operands of tcgen05.mma and tcgen05.commit stay in uniform registers, while a branch on the lane index has them moved there before every
 // instruction.

@@ -1,0 +1,277 @@
+// GEMV of one int8 activation row with GGUF-packed weights (Q4_0, Q8_0, Q4_K, Q6_K):  y[n] = sum_k W[n, k] x[k].
+//
+// Latency-mode decoding streams every weight once per token, so this kernel is a stream of packed rows through shared memory: every warp has
+// a ring of its own, filled by 16-byte asynchronous copies with up to 2048 weights of a row (1152 to 2176 bytes) per slot, and takes rows of
+// the grid's order one after the other. The ring is filled before the wait for the previous kernel: the weights do not depend
+// on it. Blocks are read from shared memory with the word accesses their alignment there allows (16 bytes for Q4_K; words of 2-byte
+// aligned blocks are joined by a byte permutation), multiplied with the int8 activations by dp4a, and scaled in fp32 as in quant_ops.cu.
+// The activations lie in shared memory too: read from global memory by lanes 64 bytes apart they took four times as many cycles of the
+// L1 port as the weights. One warp per row with loads of single blocks from global memory (quant_ops.cu): a token of four 8B layers
+// and the head in Q4_K_M 436 us, with this kernel 371; 22 layers of 1.1B in Q4_0 752 and 719. What bounds it: the instructions of a
+// chunk, about three per weight and lane (28672 x 4096 of Q4_K: 22 us, 3.0 TB/s; 128256 x 4096 of Q6_K: 124 us, 3.5 TB/s).
+#include "quant_ops.cuh"
+
+#include "../common/device_info.h"
+#include "../common/sm100.cuh"
+#include "quant_blocks.cuh"
+
+namespace oxb {
+
+namespace {
+
+constexpr int kWarps = 8;
+constexpr int kChunk = 2048;                  // weights of a row per ring slot
+constexpr int kSlots = 4;                     // per warp; with the activations of 28672 values two CTAs fit on an SM
+
+__host__ __device__ constexpr int slot_bytes(int type) {  // of kChunk weights
+  return type == kQ_Q8_0 ? 2176 : (type == kQ_Q6_K ? 1680 : 1152);
+}
+
+__device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void* gsrc) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ float half_of(uint32_t bits) { return __half2float(__ushort_as_half(static_cast<uint16_t>(bits & 0xFFFFu))); }
+__device__ __forceinline__ float to_float(int v) {  // |v| < 2^22, two full-rate instructions
+  return __int_as_float(0x4B400000 + v) - 12582912.f;
+}
+// N words from the 2-byte aligned address `p` in shared memory.
+template <int N>
+__device__ __forceinline__ void words_a2(const uint8_t* p, uint32_t (&w)[N]) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
+  const uint32_t sel = (a & 2) ? 0x5432u : 0x3210u;
+  uint32_t r[N + 1];
+#pragma unroll
+  for (int i = 0; i <= N; ++i) r[i] = q[i];
+#pragma unroll
+  for (int i = 0; i < N; ++i) w[i] = __byte_perm(r[i], r[i + 1], sel);
+}
+__device__ __forceinline__ int dot4(const uint32_t* w, int4 x, int s) {
+  s = __dp4a(static_cast<int>(w[0]), x.x, s);
+  s = __dp4a(static_cast<int>(w[1]), x.y, s);
+  s = __dp4a(static_cast<int>(w[2]), x.z, s);
+  return __dp4a(static_cast<int>(w[3]), x.w, s);
+}
+
+// The activation row in shared memory: 16-byte units, unit i at i ^ (i / 8 % 8) of its 128-byte line's place, so that lanes that read units 2 or
+// 4 apart meet in no bank; then (scale, scaled sum) of every 32 values.
+struct Row8 {
+  const int4* x;
+  const float2* ds;
+};
+__device__ __forceinline__ int unit_place(int i) { return i ^ ((i >> 3) & 7); }
+
+// One group of 32 weights, as words of four signed codes with the scales of its halves and an offset.
+__device__ __forceinline__ float group_dot(const Row8& a, int grp, const uint32_t (&w)[8], float dl0, float dl1, float ml) {
+  const int lo = dot4(w, a.x[unit_place(2 * grp)], 0), hi = dot4(w + 4, a.x[unit_place(2 * grp + 1)], 0);
+  const float2 ds = a.ds[grp];
+  return ds.x * (dl0 * to_float(lo) + dl1 * to_float(hi)) + ml * ds.y;
+}
+
+// The warp's share of a chunk of `n_sb` super-blocks (256 weights) that starts at `s` and is number `sb0` of its row on.
+template <int T>
+__device__ __forceinline__ float chunk_dot(const Row8& a, const uint8_t* s, int sb0, int n_sb, int lane) {
+  float acc = 0.f;
+  if constexpr (T == kQ_Q4_K || T == kQ_Q6_K) {
+    const int sb = lane >> 2, j = lane & 3;  // four lanes per super-block
+    if (sb >= n_sb) return 0.f;
+    uint32_t w[2][8];
+    if constexpr (T == kQ_Q4_K) {
+      const uint8_t* b = s + sb * 144;
+      const uint4 hdr = *reinterpret_cast<const uint4*>(b);
+      const uint4 qa = reinterpret_cast<const uint4*>(b + 16)[2 * j], qb = reinterpret_cast<const uint4*>(b + 16)[2 * j + 1];
+      const uint32_t n[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        w[0][u] = n[u] & 0x0F0F0F0Fu;
+        w[1][u] = (n[u] >> 4) & 0x0F0F0F0Fu;
+      }
+      // 6-bit scales and minima of sub-blocks 2 j and 2 j + 1
+      const uint32_t sc = j < 2 ? hdr.y & 0x3F3F3F3Fu : (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
+      const uint32_t mn = j < 2 ? hdr.z & 0x3F3F3F3Fu : ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
+      const float d = half_of(hdr.x), dmin = half_of(hdr.x >> 16);
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const int sh = 8 * ((2 * j + g) & 3);
+        const float dl = d * static_cast<float>((sc >> sh) & 0xFFu);
+        acc += group_dot(a, (sb0 + sb) * 8 + 2 * j + g, w[g], dl, dl, -dmin * static_cast<float>((mn >> sh) & 0xFFu));
+      }
+    } else {
+      // bytes [32 (j & 1), ..) of half j / 2: low nibbles are quarter j & 1, high ones quarter 2 + (j & 1)
+      const uint8_t* b = s + sb * 210;
+      const int half = j >> 1, first = j & 1;
+      uint32_t l[8], h[8];
+      words_a2<8>(b + half * 64 + first * 32, l);
+      words_a2<8>(b + 128 + half * 32, h);
+      const float d = half_of(*reinterpret_cast<const uint16_t*>(b + 208));
+      const int hs = 2 * first;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        // code - 32 per byte, no borrow between bytes: (code | 128) - 32, then the top bit back
+        const uint32_t v = (l[u] & 0x0F0F0F0Fu) | (((h[u] >> hs) << 4) & 0x30303030u) | 0x80808080u;
+        const uint32_t c = ((l[u] >> 4) & 0x0F0F0F0Fu) | ((h[u] >> hs) & 0x30303030u) | 0x80808080u;
+        w[0][u] = (v - 0x20202020u) ^ 0x80808080u;
+        w[1][u] = (c - 0x20202020u) ^ 0x80808080u;
+      }
+#pragma unroll
+      for (int g = 0; g < 2; ++g) {
+        const int quarter = first + 2 * g;
+        const uint32_t sc = *reinterpret_cast<const uint16_t*>(b + 192 + half * 8 + quarter * 2);
+        acc += group_dot(a, (sb0 + sb) * 8 + half * 4 + quarter, w[g], d * static_cast<float>(static_cast<int8_t>(sc & 0xFF)),
+                         d * static_cast<float>(static_cast<int8_t>(sc >> 8)), 0.f);
+      }
+    }
+  } else {
+    // two blocks of 32 per lane
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int g = lane + 32 * i;
+      if (g >= n_sb * 8) break;
+      uint32_t w[8];
+      if constexpr (T == kQ_Q4_0) {
+        const uint8_t* b = s + g * 18;
+        uint32_t n[4];
+        words_a2<4>(b + 2, n);
+        const float d = half_of(*reinterpret_cast<const uint16_t*>(b));
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          w[u] = n[u] & 0x0F0F0F0Fu;
+          w[4 + u] = (n[u] >> 4) & 0x0F0F0F0Fu;
+        }
+        acc += group_dot(a, sb0 * 8 + g, w, d, d, -8.f * d);
+      } else {
+        const uint8_t* b = s + g * 34;
+        words_a2<8>(b + 2, w);
+        const float d = half_of(*reinterpret_cast<const uint16_t*>(b));
+        acc += group_dot(a, sb0 * 8 + g, w, d, d, 0.f);
+      }
+    }
+  }
+  return acc;
+}
+
+// Row (r * gridDim.x + CTA) * 8 + warp in round r.
+__global__ void __launch_bounds__(kWarps * 32, 2) gemv_packed_kernel(const MmvqParams p, const int slot_size) {
+  extern __shared__ __align__(128) uint8_t s_mem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunks = (p.K + kChunk - 1) / kChunk, groups = p.K >> 5;
+  int4* s_x = reinterpret_cast<int4*>(s_mem);
+  float2* s_ds = reinterpret_cast<float2*>(s_mem + p.K);
+  uint8_t* ring = s_mem + p.K + groups * 8 + warp * kSlots * slot_size;
+
+  // rows of this warp: n, n + step, ...
+  const int step = static_cast<int>(gridDim.x) * kWarps;
+  struct Row {
+    const uint8_t* w;
+    int type, n;
+    long long bytes;
+  };
+  auto find = [&](Row& x) {  // the segment of row x.n
+    int seg = 0, row0 = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (seg == i && i + 1 < p.n_seg && x.n >= p.seg_row_end[i]) {
+        row0 = p.seg_row_end[i];
+        seg = i + 1;
+      }
+    x.type = p.seg_type[seg];
+    x.bytes = p.seg_row_bytes[seg];
+    x.w = p.seg_w[seg] + static_cast<long long>(x.n - row0) * x.bytes;
+  };
+  auto next = [&](Row& x) {
+    x.n += step;
+    if (p.n_seg == 1) x.w += step * x.bytes;
+    else if (x.n < p.N) find(x);
+  };
+  Row row{nullptr, 0, static_cast<int>(blockIdx.x) * kWarps + warp, 0};
+  if (row.n < p.N) find(row);
+
+  // ---- requests run kSlots chunks ahead of the products; one group of copies per chunk, empty ones behind the last ----
+  int ic = 0, is = 0;
+  Row irow = row;
+  auto request = [&]() {
+    if (irow.n < p.N) {
+      const int sb = p.K - ic * kChunk < kChunk ? (p.K - ic * kChunk) >> 8 : kChunk >> 8;
+      const int bytes = sb * (slot_bytes(irow.type) / 8);
+      const uint8_t* src = irow.w + static_cast<long long>(ic) * slot_bytes(irow.type);
+      const uint32_t dst = smem_u32(ring + is * slot_size);
+#pragma unroll
+      for (int i = 0; i < 5; ++i)  // 2176 bytes at most
+        if ((lane + 32 * i) * 16 < bytes) cp_async_16(dst + (lane + 32 * i) * 16, src + (lane + 32 * i) * 16);
+      if (++is == kSlots) is = 0;
+      if (++ic == chunks) {
+        ic = 0;
+        next(irow);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i < kSlots; ++i) request();
+  pdl_wait();  // the activation row comes from the kernel before this one
+  for (int i = threadIdx.x; i < p.K >> 4; i += kWarps * 32) s_x[unit_place(i)] = __ldg(reinterpret_cast<const int4*>(p.xq) + i);
+  for (int i = threadIdx.x; i < groups; i += kWarps * 32) s_ds[i] = make_float2(__ldg(p.xd + i), __ldg(p.xs + i));
+  __syncthreads();
+  const Row8 x8 = {s_x, s_ds};
+
+  int cs = 0;
+  for (; row.n < p.N; next(row)) {
+    float acc = 0.f;
+    for (int c = 0; c < chunks; ++c) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 1) : "memory");
+      __syncwarp();  // the copies of all lanes have landed
+      const uint8_t* s = ring + cs * slot_size;
+      const int n_sb = p.K - c * kChunk < kChunk ? (p.K - c * kChunk) >> 8 : kChunk >> 8;
+      switch (row.type) {
+        case kQ_Q4_0: acc += chunk_dot<kQ_Q4_0>(x8, s, c * 8, n_sb, lane); break;
+        case kQ_Q8_0: acc += chunk_dot<kQ_Q8_0>(x8, s, c * 8, n_sb, lane); break;
+        case kQ_Q4_K: acc += chunk_dot<kQ_Q4_K>(x8, s, c * 8, n_sb, lane); break;
+        default: acc += chunk_dot<kQ_Q6_K>(x8, s, c * 8, n_sb, lane); break;
+      }
+      __syncwarp();  // every lane has read the slot
+      request();
+      if (++cs == kSlots) cs = 0;
+    }
+    if (row.n + step >= p.N) pdl_launch_dependents();  // the weight stream is done: the next kernel may become resident
+    float v = warp_sum(acc);
+    if (lane != 0) continue;
+    if (p.bias != nullptr) v += __bfloat162float(p.bias[row.n]);
+    if (p.out_f32 != nullptr) {
+      p.out_f32[row.n] = p.add ? p.out_f32[row.n] + v : v;
+    } else {
+      if (p.add) v += __bfloat162float(p.out_bf16[row.n]);
+      p.out_bf16[row.n] = __float2bfloat16(v);
+    }
+  }
+}
+
+}  // namespace
+
+bool gemv_packed_takes(const MmvqParams& p) {
+  // One row: with more the products bound it, not the stream. The copies want 16-byte aligned rows of a multiple of 16 bytes (Q6_K: K a
+  // multiple of 2048); a chunk is that for every type. The activations of 28672 values leave room for two CTAs per SM.
+  if (p.M != 1 || p.N < 1 || p.K < 256 || p.K > 28672 || p.K % 256 != 0 || p.xq == nullptr || p.xd == nullptr || p.xs == nullptr) return false;
+  if (reinterpret_cast<uintptr_t>(p.xq) % 16 != 0) return false;
+  for (int i = 0; i < p.n_seg; ++i) {
+    const int t = p.seg_type[i];
+    if (t != kQ_Q4_0 && t != kQ_Q8_0 && t != kQ_Q4_K && t != kQ_Q6_K) return false;
+    if (reinterpret_cast<uintptr_t>(p.seg_w[i]) % 16 != 0 || p.seg_row_bytes[i] % 16 != 0) return false;
+  }
+  return p.n_seg >= 1;
+}
+
+void launch_gemv_packed(const MmvqParams& p, cudaStream_t stream) {
+  int slot_size = 0;  // 16 bytes more than a chunk: words are read in pairs
+  for (int i = 0; i < p.n_seg; ++i) {
+    const int need = slot_bytes(p.seg_type[i]) + 16;
+    slot_size = need > slot_size ? need : slot_size;
+  }
+  // as few rounds as two CTAs per SM allow, then as few CTAs as those rounds need
+  const int per_round = 2 * sm_count() * kWarps;
+  const int rounds = (p.N + per_round - 1) / per_round;
+  const int grid = (p.N + rounds * kWarps - 1) / (rounds * kWarps);
+  const size_t smem = static_cast<size_t>(kWarps) * kSlots * slot_size + p.K + static_cast<size_t>(p.K / 32) * 8;
+  ensure_dynamic_smem(gemv_packed_kernel, smem);
+  launch_kernel(gemv_packed_kernel, dim3(grid), dim3(kWarps * 32), smem, stream, /*pdl=*/true, false, p, slot_size);
+}
+
+}  // namespace oxb

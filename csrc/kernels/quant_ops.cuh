@@ -42,6 +42,10 @@ bool launch_mmvq(int qtype, const MmvqParams& p, cudaStream_t stream);
 // Q | K | V or gate | up projections of a mixed-precision GGUF file). Needs the int8 activations
 // (xq / xd / xs). Returns false when a segment's type has no integer path or an operand is misaligned.
 bool launch_mmvq_mixed(const MmvqParams& p, cudaStream_t stream);
+// One int8 row, types and alignments whose packed rows can be streamed through shared memory (gemv_packed.cu); segments as for
+// launch_mmvq_mixed, at least one.
+bool gemv_packed_takes(const MmvqParams& p);
+void launch_gemv_packed(const MmvqParams& p, cudaStream_t stream);
 bool launch_dequant_rows(int qtype, const uint8_t* w, long long row_bytes, const int* row_ids,
                          int n_rows, int K, __nv_bfloat16* out, long long ldo, float scale,
                          int n_src_rows, cudaStream_t stream);

@@ -50,7 +50,7 @@ HYBRID_KERNELS = ("stream_ops.cu", "mixer_ops.cu", "attn_rows.cu", "retention.cu
 HYBRID_HEADERS = ("hybrid.cuh", "hybrid_dev.cuh", "hybrid_mma.cuh")
 SHARED_HEADERS = ("attn.cuh", "attn_prefill_tc.cuh")   # of both kernel extensions
 # kernels of the extension that only quantised weights load
-QUANT_KERNELS = ("quant_ops.cu", "gemm_fp8_block.cu", "nvfp4_quant.cu")
+QUANT_KERNELS = ("quant_ops.cu", "gemv_packed.cu", "gemm_fp8_block.cu", "nvfp4_quant.cu")
 
 
 def _sources(name: str) -> list[Path]:

@@ -758,6 +758,54 @@ def test_dequant_and_mmvq(ops, qname):
     assert _rel_err(yb, x.float() @ ref.T + bias.float() + y0.float()) < 2e-2
 
 
+@pytest.mark.parametrize("qname", ["Q4_0", "Q8_0", "Q4_K", "Q6_K"])
+@pytest.mark.parametrize("n,k", [(1, 2048), (77, 2048), (2560, 2048), (2369, 6144), (40000, 2048), (9, 28672), (300, 256), (513, 5632), (33, 2304)])
+def test_gemv_of_streamed_rows(ops, qname, n, k):
+    """One to three int8 rows (one: packed rows streamed through shared memory), partial chunks, one row per grid and many rounds, results
+    added to what is there, against the exact product of the int8 activations with the decoded weights (32-bit sums)."""
+    from oxide_tech_llm_engine_b200.formats import quants
+    from oxide_tech_llm_engine_b200.models.llama import random_quant_linear
+
+    gen = torch.Generator(device=DEV).manual_seed(n + k)
+    lin = random_quant_linear(qname, n, k, torch.device(DEV), gen)
+    rows = lin.w.cpu().numpy().reshape(n, -1)
+    decoded = lambda raw: torch.from_numpy(quants.dequantize_2d(qname, np.ascontiguousarray(raw), len(raw), k)).to(DEV).double()
+    some, last = decoded(rows[:64]), decoded(rows[-1:])
+    for m, add in ((1, False), (1, True), (3, True)):
+        x = torch.randn(m, k, device=DEV, generator=gen).to(torch.bfloat16)
+        q8, xd, xs = ops.quant_q8_1(x)
+        deq = (q8.double().view(m, k // 32, 32) * xd.double()[..., None]).view(m, k)
+        y = torch.full((m, n + 5), 3.0, device=DEV)
+        ops.mmvq(lin.code, lin.w, x, y[:, :n], n=n, k=k, add=add, xq=(q8, xd, xs))
+        torch.cuda.synchronize()
+        off = 3.0 if add else 0.0
+        for w, got in ((some, y[:, :min(n, 64)]), (last, y[:, n - 1:n])):
+            ref = deq @ w.T
+            bound = 1e-5 * (deq.abs() @ w.abs().T) + 1e-6   # products and offsets of a block cancel: relative to their sizes
+            assert ((got.double() - off - ref).abs() <= bound).all(), (m, (got.double() - off - ref).abs().max())
+        assert (y[:, n:] == 3.0).all()
+
+
+def test_gemv_of_streamed_rows_of_several_types(ops):
+    """Q|K|V of a mixed file in one launch: rows of three matrices of two block types, the same sums as one by one."""
+    from oxide_tech_llm_engine_b200.models.llama import random_quant_linear
+
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    k, parts = 4096, [("Q4_K", 4096), ("Q4_K", 1024), ("Q6_K", 1029)]
+    lins = [random_quant_linear(t, n, k, torch.device(DEV), gen) for t, n in parts]
+    x = torch.randn(1, k, device=DEV, generator=gen).to(torch.bfloat16)
+    xq = ops.quant_q8_1(x)
+    got = torch.zeros(1, sum(n for _, n in parts), device=DEV)
+    ops.mmvq_mixed([(q.code, q.w, q.n) for q in lins], x, got, k=k, xq=xq)
+    want = torch.zeros_like(got)
+    at = 0
+    for q in lins:
+        ops.mmvq(q.code, q.w, x, want[:, at:at + q.n], n=q.n, k=k, xq=xq)
+        at += q.n
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("qname", ["Q4_K", "Q6_K", "Q8_0", "Q5_K", "Q5_0", "Q4_0", "Q4_1", "Q5_1"])
 def test_gemm_with_gguf_weights_unpacked_in_the_kernel(ops, qname):
     """tcgen05 GEMM whose weight operand stays GGUF-packed in HBM: against fp32 of the activations times
