@@ -447,11 +447,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    // NVFP4: the whole warp walks and waits, an elected lane issues (elect_one: the operands stay in uniform registers; expert products of
-    // 128 rows 269 -> 252 us). The bf16 products outlast the issue of one thread (with 256 rows a step is 1 % slower that way).
-    constexpr bool kWarpIssue = FP4;
-    if (kWarpIssue || lane == 0) {
-      constexpr uint32_t idesc = make_idesc(kFmtBF16, kFmtBF16, BM, BN);
+    if constexpr (FP4) {
+      // The whole warp walks and waits, an elected lane issues (elect_one: the operands stay in uniform registers): expert products of
+      // 128 rows 269 -> 252 us. The bf16 products below outlast the issue of one thread, and nothing is faster for them that way.
+      constexpr uint32_t idesc4 = make_idesc_nvfp4(BM, BN);
       uint32_t iter = 0, s = 0, ph = 0, t = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
@@ -464,41 +463,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const uint32_t d_tmem = tmem_base + buf * kItemCols;
         for (int kb = 0; kb < it.nkb; ++kb, ++iter) {
           if (ok && !mbar_wait(&full[s], ph, spin)) ok = false;
-          if (kWarpIssue) ok = __all_sync(0xffffffffu, ok);
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after_sync();
           const uint32_t a_addr = smem_u32(sA + s * L::kABytes);
           const uint32_t b_addr = smem_u32(sB + s * L::kBBytes);
-          if (!kWarpIssue || elect_one()) {
-            if constexpr (FP4) {
-              // scales of this k block -> TMEM (alternating column sets), then 4 MMAs of 64 values of K
-              constexpr uint32_t idesc4 = make_idesc_nvfp4(BM, BN);
-              const uint32_t sfa_t = tmem_base + kSFCol0 + (iter & 1) * 32;
-              const uint32_t sfb_t = sfa_t + 16;
-              const uint32_t sf_s = smem_u32(sSF + s * (L::kSFABytes + L::kSFBBytes));
+          // scales of this k block -> TMEM (alternating column sets), then 4 MMAs of 64 values of K
+          const uint32_t sfa_t = tmem_base + kSFCol0 + (iter & 1) * 32;
+          const uint32_t sfb_t = sfa_t + 16;
+          const uint32_t sf_s = smem_u32(sSF + s * (L::kSFABytes + L::kSFBBytes));
+          if (elect_one()) {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                tc_cp_scales(sfa_t + 4 * j, make_desc_scales(sf_s + j * 512));
-                tc_cp_scales(sfb_t + 4 * j, make_desc_scales(sf_s + L::kSFABytes + j * 512));
-              }
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                tc_mma_nvfp4(d_tmem, make_desc_kmajor_sw128(a_addr + k * 32), make_desc_kmajor_sw128(b_addr + k * 32),
-                             idesc4, (kb | k) != 0 ? 1u : 0u, sfa_t + 4 * k, sfb_t + 4 * k);
-            } else {
-#pragma unroll
-              for (int k = 0; k < BK / 16; ++k) {
-                const uint64_t db = make_desc_kmajor_sw128(b_addr + k * 32);
-#pragma unroll
-                for (int h = 0; h < MT; ++h)
-                  tc_mma_f16(d_tmem + h * kAccCols, make_desc_kmajor_sw128(a_addr + h * (BM * BK * 2) + k * 32),
-                             db, idesc, (kb | k) != 0 ? 1u : 0u);
-              }
+            for (int j = 0; j < 4; ++j) {
+              tc_cp_scales(sfa_t + 4 * j, make_desc_scales(sf_s + j * 512));
+              tc_cp_scales(sfb_t + 4 * j, make_desc_scales(sf_s + L::kSFABytes + j * 512));
             }
-            tc_commit(&empty[s]);  // frees this smem stage once the MMAs above have read it
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              tc_mma_nvfp4(d_tmem, make_desc_kmajor_sw128(a_addr + k * 32), make_desc_kmajor_sw128(b_addr + k * 32),
+                           idesc4, (kb | k) != 0 ? 1u : 0u, sfa_t + 4 * k, sfb_t + 4 * k);
+            tc_commit(&empty[s]);
             if (kb == it.nkb - 1) tc_commit(&tmem_full[buf]);
           }
-          if (kWarpIssue) __syncwarp();
+          __syncwarp();
           if (++s == STAGES) {
             s = 0;
             ph ^= 1;
@@ -508,6 +495,48 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       if (!ok && lane == 0) set_status_once(p.status, kStatusMbarTimeoutMma);
       if (lane == 0) pdl_launch_dependents();  // only epilogues are left in this CTA
+    } else if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(kFmtBF16, kFmtBF16, BM, BN);
+      uint32_t iter = 0, t = 0;
+      bool ok = true;
+      for (int w = blockIdx.x; w < n_work && ok; w += gridDim.x) {
+        const WorkItem it = decode(w);
+        if (!it.valid) continue;
+        const uint32_t buf = t % kBufs;
+        const uint32_t use = t / kBufs;
+        // the epilogue must have drained this accumulator buffer (kBufs items ago)
+        if (use >= 1 && !mbar_wait(&tmem_empty[buf], (use & 1) ^ 1, spin)) {
+          set_status_once(p.status, kStatusMbarTimeoutMma);
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+        const uint32_t d_tmem = tmem_base + buf * kItemCols;
+        for (int kb = 0; kb < it.nkb; ++kb, ++iter) {
+          const int s = iter % STAGES;
+          const uint32_t ph = (iter / STAGES) & 1;
+          if (!mbar_wait(&full[s], ph, spin)) {
+            set_status_once(p.status, kStatusMbarTimeoutMma);
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+          const uint32_t a_addr = smem_u32(sA + s * L::kABytes);
+          const uint32_t b_addr = smem_u32(sB + s * L::kBBytes);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) {
+            const uint64_t db = make_desc_kmajor_sw128(b_addr + k * 32);
+#pragma unroll
+            for (int h = 0; h < MT; ++h)
+              tc_mma_f16(d_tmem + h * kAccCols, make_desc_kmajor_sw128(a_addr + h * (BM * BK * 2) + k * 32),
+                         db, idesc, (kb | k) != 0 ? 1u : 0u);
+          }
+          tc_commit(&empty[s]);  // frees this smem stage once the MMAs above have read it
+        }
+        if (ok) tc_commit(&tmem_full[buf]);
+        ++t;
+      }
+      pdl_launch_dependents();  // only epilogues are left in this CTA
     }
   } else if (PACKED && warp >= 6) {
     // ------------------------------ weight unpacking (KIND 2) -----------------
