@@ -252,7 +252,7 @@ void gemm_bf16(const Tensor& a, const Tensor& w, int64_t epi, const c10::optiona
     p.ws = reinterpret_cast<__nv_bfloat16*>(ws->data_ptr());
     p.ws_tickets = reinterpret_cast<uint32_t*>(ws_tickets->data_ptr());
   }
-  if (oxb::gemm_pair_takes(p, mt_i)) {
+  if (oxb::gemm_pair_takes(p, bn_i, mt_i)) {
     const CUtensorMap tmB128 =
         tiled ? oxb::make_tma_map(w.data_ptr(), dt, 2, 3, 64, 128, static_cast<uint64_t>(w.size(0) * w.size(1)), 128, 16384, 64, 128,
                                   1, CU_TENSOR_MAP_SWIZZLE_128B)

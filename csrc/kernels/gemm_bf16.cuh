@@ -109,8 +109,8 @@ void launch_gemm_bf16(const CUtensorMap& tmA, const CUtensorMap& tmB, const Gemm
                       int mt, cudaStream_t stream);
 
 // The GEMM of CTA pairs (gemm_pair.cu): 256 x 256 tiles, maps with boxes of 128 rows. `gemm_pair_takes` says whether a
-// launch with these parameters has enough rows and tiles for it and asks for nothing that it does not do.
-bool gemm_pair_takes(const GemmParams& p, int mt);
+// launch with these parameters (and, on the general kernel, tiles of bn columns) has enough rows and tiles for it and asks for nothing that it does not do.
+bool gemm_pair_takes(const GemmParams& p, int bn, int mt);
 void launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream);
 
 // Activation quantiser of the NVFP4 GEMM: bf16 rows -> packed e2m1 + ue4m3 block scales (atom layout

@@ -325,7 +325,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 }  // namespace
 
-bool gemm_pair_takes(const GemmParams& p, int mt) {
+bool gemm_pair_takes(const GemmParams& p, int bn, int mt) {
   // one GPU's own rows, whole K: what needs flags, peers, splits or other operands stays with gemm_bf16.cu
   if (p.kind != 0 || mt != 1 || p.splits != 1 || p.ag_flags != nullptr || p.trace != nullptr || p.epi == kEpiSlabBf16) return false;
   if (p.epi == kEpiRedF32) {
@@ -339,7 +339,14 @@ bool gemm_pair_takes(const GemmParams& p, int mt) {
   if (p.n_groups > 0 && p.group_counts == nullptr) return p.M >= kTile && p.n_groups * ((p.M + kTile - 1) / kTile) * n_tiles >= pairs;
   // grouped: m_tiles bounds the 128-row tiles of all groups, one unfinished tile per group included
   if (p.n_groups > 0) return p.m_tiles - p.n_groups >= 2 * p.n_groups && (p.m_tiles - p.n_groups) / 2 * n_tiles >= pairs;
-  return p.M > kTile && (p.M + kTile - 1) / kTile * n_tiles >= pairs;
+  // Rounds of the chip: a last row tile that is mostly padding, or a second round for a few tiles, can cost more than the pairs save. Up to
+  // 1500 rows a round of the general kernel with tiles of 256 columns takes 1.1 to 1.25 times one of pairs, with 128 columns three
+  // quarters of that. 257 / 400 / 770 rows, 10240 x 8192: 71 / 121 / 121 us there, 125 / 99 / 141 here; 11264 x 2048: 27 / 40 / 53 and
+  // 33 / 33 / 45.
+  const int tiles = (p.M + kTile - 1) / kTile * n_tiles;
+  const int others = (p.M + kHalf - 1) / kHalf * ((p.N + bn - 1) / bn);
+  const int rounds = (tiles + pairs - 1) / pairs, other_rounds = (others + sm_count() - 1) / sm_count();
+  return p.M > kTile && tiles >= pairs && rounds * 1024 <= other_rounds * (kHalf + bn) * 3;
 }
 
 void launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, cudaStream_t stream) {
